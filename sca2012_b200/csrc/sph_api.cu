@@ -280,6 +280,17 @@ template <int DIM> void hash_prologue(sph_handle *h)
     h->last_launches += 1;
 }
 
+// The density pass with its buffers in dynamic shared memory (above 48 KB, the
+// 512-thread shape, only after the kernel's limit is raised).
+template <int DIM, int B, bool SKIP>
+void launch_density(sph_handle *h, uint32_t grid, Counters *cin, const WorkPtrs &w)
+{
+    auto kern = k_density<DIM, B, SKIP>;
+    if (kDensSmemBytes<B> > (48u << 10))
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDensSmemBytes<B>);
+    kern<<<grid, B, kDensSmemBytes<B>, h->stream>>>(h->cfg, cin, w);
+}
+
 // One step as separate launches.  prologue = false leaves out the hash of a
 // state no step has hashed (a captured graph: the replay runs it when needed).
 template <int DIM> int run_step(sph_handle *h, bool prologue = true)
@@ -315,9 +326,9 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
     stage(h, "reorder");
     const uint32_t gd = grid_st(h, nub, SPH_TUNE_DENSITY);
     if (c.density_skip_r2 == 0.0f) {
-        SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_DENSITY], k_density<DIM, B, false><<<gd, B, 0, s>>>(c, cin, w));
+        SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_DENSITY], launch_density<DIM, B, false>(h, gd, cin, w));
     } else {
-        SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_DENSITY], k_density<DIM, B, true><<<gd, B, 0, s>>>(c, cin, w));
+        SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_DENSITY], launch_density<DIM, B, true>(h, gd, cin, w));
     }
     stage(h, "density");
     SPH_BS_SWITCH2(h->tune_bs[SPH_TUNE_FORCE], h->tune_minb[SPH_TUNE_FORCE],

@@ -29,6 +29,7 @@
 // rounds the same way and the two give the same bits.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include "../../include/sph/sph.h"
 
 namespace sph {
@@ -177,6 +178,17 @@ __device__ __forceinline__ uint3 cell_of(const sph_config &c, float4 p)
 __device__ __forceinline__ uint32_t key_of(const sph_config &c, uint32_t x, uint32_t y, uint32_t z)
 {
     return z * c.ncell[0] * c.ncell[1] + y * c.ncell[0] + x;
+}
+
+// The cell coordinates of a key (two integer divisions).
+template <int DIM> __device__ __forceinline__ uint3 cell_of_key(const sph_config &c, uint32_t k)
+{
+    uint3 q;
+    const uint32_t yz = k / c.ncell[0];
+    q.x = k - yz * c.ncell[0];
+    q.z = DIM == 3 ? yz / c.ncell[1] : 0u;
+    q.y = DIM == 3 ? yz - q.z * c.ncell[1] : yz;
+    return q;
 }
 
 // fma(dz, dz, fma(dx, dx, dy*dy)) with d = a - b, all round-to-nearest.
@@ -416,83 +428,237 @@ __device__ __forceinline__ void warp_pairs(const sph_config &c, const uint32_t *
 // ------------------------------------------------------------ 5. density
 // rho_i = m_i poly6_i h_i^6 + sum_{j != i, skip <= r^2 < h_i^2} m_j poly6_i (h_i^2 - r^2)^3
 // p_i = k ((rho_i / rho0)^3 - 1)         (SPH-3D-2/sph_system.cu:338-677)
+// The walk's inner loop is the distance test alone, on candidates staged in
+// shared memory.  A warp's 32 particles lie in a few neighbouring cells, so
+// their ranges of a stencil row overlap: the warp stages the row 64 slots at a
+// time (each lane loads two, a chunk ahead of its use), laid out in pairs so
+// that one packed FP32 instruction serves two candidates, and each lane tests
+// its own range of it.  A candidate within (1 + margin) h_max goes, with its
+// r^2, to the lane's column of a small buffer.  The warp drains its buffers
+// together: each lane adds its buffered pairs into its own density sum in walk
+// order (to the bit the sum of a walk that adds as it goes) and stores the
+// slots to its candidate list in whole chunks of four.
+// Bound: the L1 / shared-memory data pipe (77 % of its wavefronts) beside
+// instruction issue (66 %).  A 16-byte global load costs the pipe at least 4
+// wavefronts however many lanes share its address, a staged one 2 to 3; a
+// walk that loaded each candidate from global memory, summed it at once and
+// stored its slot with a 4-byte store of its own held the pipe at 83 %.
+// 1.24M particles (four-way dam): 0.358 -> 0.287 ms; 1.05M without splits:
+// 0.222 -> 0.177 ms.
+constexpr uint32_t kDensLevel2 = 1u << 30;   // in a staged slot number: not level 1 (max_particle <= 2^30)
+
+// CAP buffer entries per lane (entry-major: appends and reads hit distinct
+// banks), and the staged chunk: pair p holds slots 2p and 2p + 1.
+template <uint32_t CAP> struct DensSmem {
+    uint2 ent[CAP][32];   // (r^2, tagged slot)
+    float4 xy[34];        // (x0, x1, y0, y1); the last two are read past, never used
+    uint4 zs[34];         // (z0, tagged slot 0, z1, tagged slot 1)
+};
+
 // SKIP = false: the config skips no close pairs (density_skip_r2 == 0), so
 // the test !(r^2 < skip) is true for every r^2 and is left out.
-template <int DIM, bool NC, bool SKIP>
-__device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt, const WorkPtrs &w)
+// FLUSH: the buffer entries a warp keeps free for its next chunk.
+template <int DIM, int BS, bool NC, bool SKIP, uint32_t CAP, uint32_t FLUSH>
+__device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt, const WorkPtrs &w,
+                                             DensSmem<CAP> *smem)
 {
+    const unsigned full = 0xffffffffu;
     const uint32_t n = cnt->n;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt->disp2_max = 0u;   // the force pass takes the max
-    for (uint32_t s = grid_stride_start(); s < n; s += grid_stride()) {
+    DensSmem<CAP> &sm = smem[wib];
+    uint2 *const col = &sm.ent[0][lane];
+    // the append position as a shared-memory address (256 bytes per entry)
+    const uint32_t col0 = (uint32_t)__cvta_generic_to_shared(col), col_lim = col0 + (CAP - 4) * 256u;
+    constexpr int nrows = DIM == 3 ? 9 : 3, own = nrows / 2;
+    // list entry k at lbase[(k >> 2) * row4 + (k & 3)] (nl_at; the offset
+    // fits 32 bits under the lists' 12 GB allocation limit)
+    const bool rec = w.nlist != nullptr;
+    const uint32_t row4 = w.nl_stride * 4u;
+    // warp-uniform grid-stride loop: a warp takes 32 consecutive slots
+    for (uint32_t base = blockIdx.x * BS + wib * 32u; base < n; base += gridDim.x * BS) {
+        const uint32_t s_raw = base + lane;
+        const bool valid = s_raw < n;
+        const uint32_t s = valid ? s_raw : n - 1u;
         const float4 pi = w.spos[s];
         const int li = lv(pi.w);
         const float h2 = c.kernel2[li];
         const float poly6 = c.poly6[li];
         const uint32_t k = w.skey[s];
-        uint3 q;
-        q.x = k % c.ncell[0];
-        q.y = (k / c.ncell[0]) % c.ncell[1];
-        q.z = DIM == 3 ? k / (c.ncell[0] * c.ncell[1]) : 0u;
-        float rho = 0.0f;
-        uint32_t nb = 0, nl = 0;
+        const uint3 q = cell_of_key<DIM>(c, k);
         const float m0 = c.mass[0], m1 = c.mass[1], skip = c.density_skip_r2;
-        // the force and energy passes' candidates on the way
-        // (r^2 < (1 + margin)^2 h_max^2), in the order their walks find them
-        const bool rec = w.nlist != nullptr;
-        const float re2 = energy_list_r2(c);
         // (m_j * poly6) once per level: the same product the sum takes first
         const float mp0 = m0 * poly6, mp1 = m1 * poly6;
-        // single pass: the kernel sum is cheap enough to run predicated
-        // (:394-417, j != i with skip <= r^2 < h_i^2)
-        // list entry k at lbase[(k >> 2) * row4 + (k & 3)] (nl_at; the offset
-        // fits 32 bits under the lists' 12 GB allocation limit)
+        const float reach2 = rec ? energy_list_r2(c) : h2;
+        const uint32_t self = s | (li ? kDensLevel2 : 0u);
         uint32_t *const lbase = rec ? w.nlist + (size_t)s * 4u : nullptr;
-        const uint32_t row4 = w.nl_stride * 4u;
-        // dx, dy as one packed FP32 subtraction (sm_100 f32x2; each half is the
-        // IEEE round-to-nearest x_j - x_i, so r^2 is r2_of's to the bit)
-        const float2 npi = make_float2(-pi.x, -pi.y);
-        auto add = [&](uint32_t t, float4 pj) {   // t != s (the walk skips s)
-            const float2 dxy = __fadd2_rn(make_float2(pj.x, pj.y), npi);
-            float r2 = __fmaf_rn(dxy.x, dxy.x, __fmul_rn(dxy.y, dxy.y));
-            if (DIM == 3) {
-                const float dzz = __fsub_rn(pj.z, pi.z);
-                r2 = __fmaf_rn(dzz, dzz, r2);
-            }
+        float rho = 0.0f;
+        uint32_t nb = 0, nl = 0;      // nl: entries drained so far (a multiple of 4 until the end)
+        uint32_t at = col0;           // where the next buffer entry goes
+        // one buffered pair into the sum: skip <= r^2 < h_i^2 (:394-417)
+        auto take = [&](const uint2 ent) {
+            const float r2 = __uint_as_float(ent.x);
+            const float x = h2 - r2;
+            const float x3 = x * x * x;
             if ((!SKIP || !(r2 < skip)) && r2 < h2) {
-                const float x = h2 - r2;
-                rho = __fmaf_rn(pj.w == 1.0f ? mp0 : mp1, x * x * x, rho);
+                rho = __fmaf_rn(ent.y & kDensLevel2 ? mp1 : mp0, x3, rho);
                 ++nb;
             }
-            if (rec && r2 < re2) {
-                if (nl < kNbrListCap) lbase[(nl >> 2) * row4 + (nl & 3u)] = t;
-                ++nl;
-            }
         };
-        auto range = [&](uint32_t b, uint32_t e) {
-            uint32_t t = b;
-            for (; t + 4 <= e; t += 4) {
-                const float4 p0 = ldro<NC>(w.spos + t), p1 = ldro<NC>(w.spos + t + 1),
-                             p2 = ldro<NC>(w.spos + t + 2), p3 = ldro<NC>(w.spos + t + 3);
-                add(t, p0);
-                add(t + 1, p1);
-                add(t + 2, p2);
-                add(t + 3, p3);
+        // whole chunks of four, then (last) the rest; up to three entries stay
+        // at the front of the buffer in between
+        auto drain = [&](bool last) {
+            asm volatile("" ::: "memory");   // the appends below are opaque to the compiler
+            const uint32_t fill = (at - col0) >> 8, whole = fill & ~3u;
+            for (uint32_t g = 0; g < whole; g += 4) {
+                const uint2 a0 = col[(g + 0) * 32], a1 = col[(g + 1) * 32], a2 = col[(g + 2) * 32],
+                            a3 = col[(g + 3) * 32];
+                take(a0);
+                take(a1);
+                take(a2);
+                take(a3);
+                if (rec && nl < kNbrListCap)
+                    *reinterpret_cast<uint4 *>(lbase + (nl >> 2) * row4) =
+                        make_uint4(a0.y & ~kDensLevel2, a1.y & ~kDensLevel2, a2.y & ~kDensLevel2,
+                                   a3.y & ~kDensLevel2);
+                nl += 4;
             }
-            for (; t < e; ++t) add(t, ldro<NC>(w.spos + t));
+            const uint32_t rest = fill - whole;
+            if (last) {
+                uint32_t t4[4] = {s, s, s, s};
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if ((uint32_t)u < rest) {
+                        const uint2 a = col[(whole + u) * 32];
+                        take(a);
+                        t4[u] = a.y & ~kDensLevel2;
+                    }
+                if (rec && rest && nl < kNbrListCap)
+                    *reinterpret_cast<uint4 *>(lbase + (nl >> 2) * row4) = make_uint4(t4[0], t4[1], t4[2], t4[3]);
+                nl += rest;
+            } else if (whole) {
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if ((uint32_t)u < rest) col[u * 32] = col[(whole + u) * 32];
+            }
+            at = col0 + rest * 256u;
         };
-#pragma unroll 1
-        for (int dz = (DIM == 3 ? -1 : 0); dz <= (DIM == 3 ? 1 : 0); ++dz)
-#pragma unroll 1
-            for (int dy = -1; dy <= 1; ++dy) {
-                uint32_t b, e;
-                if (!row_range<DIM, NC>(c, w.cell_off, q, dy, dz, b, e)) continue;
-                if (dy == 0 && dz == 0) {   // the particle's own row: around its slot
-                    range(b, s);
-                    range(s + 1u, e);
-                } else {
-                    range(b, e);
+        const float2 nx = make_float2(-pi.x, -pi.x), ny = make_float2(-pi.y, -pi.y);
+        // slots 2p .. 2p + 3 of the staged chunk: thr0: the bound of the first
+        // (-1 when it lies before the lane's range); left: slots of the range
+        // from 2p on.  r^2 is r2_of's to the bit, two candidates per
+        // instruction (d = x_j + (-x_i) is the IEEE x_j - x_i).
+        auto quad = [&](uint32_t i, float thr0, int left, auto OWN) {
+            float r2[4];
+            uint32_t id[4];
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+                const float4 a = sm.xy[(i + u) >> 1];
+                const uint4 b = sm.zs[(i + u) >> 1];
+                const float2 dx = __fadd2_rn(make_float2(a.x, a.y), nx), dy = __fadd2_rn(make_float2(a.z, a.w), ny);
+                const float2 d2 = __ffma2_rn(dx, dx, __fmul2_rn(dy, dy));
+                r2[u] = d2.x;
+                r2[u + 1] = d2.y;
+                if (DIM == 3) {
+                    const float dz0 = __fsub_rn(__uint_as_float(b.x), pi.z), dz1 = __fsub_rn(__uint_as_float(b.z), pi.z);
+                    r2[u] = __fmaf_rn(dz0, dz0, d2.x);
+                    r2[u + 1] = __fmaf_rn(dz1, dz1, d2.y);
                 }
+                id[u] = b.y;
+                id[u + 1] = b.w;
             }
+            // predicated append: if (in range && r^2 < bound [&& not self])
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float thr = u == 0 ? thr0 : reach2;
+                if (OWN.value)
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, %5;\n\t"
+                                 "setp.lt.and.f32 p, %1, %4, p;\n\tsetp.ne.and.u32 p, %2, %6, p;\n\t"
+                                 "@p st.shared.v2.b32 [%0], {%1, %2};\n\t@p add.u32 %0, %0, 256;\n\t}"
+                                 : "+r"(at) : "f"(r2[u]), "r"(id[u]), "r"(left), "f"(thr), "r"(u), "r"(self));
+                else if (u == 0)
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, %3;\n\t"
+                                 "@p st.shared.v2.b32 [%0], {%1, %2};\n\t@p add.u32 %0, %0, 256;\n\t}"
+                                 : "+r"(at) : "f"(r2[u]), "r"(id[u]), "f"(thr));
+                else
+                    asm volatile("{\n\t.reg .pred p;\n\tsetp.gt.s32 p, %3, %5;\n\t"
+                                 "setp.lt.and.f32 p, %1, %4, p;\n\t"
+                                 "@p st.shared.v2.b32 [%0], {%1, %2};\n\t@p add.u32 %0, %0, 256;\n\t}"
+                                 : "+r"(at) : "f"(r2[u]), "r"(id[u]), "r"(left), "f"(thr), "r"(u));
+            }
+        };
+        // the lane's slot range of row r: cells x - 1 .. x + 1 (inside the
+        // grid) of row (dy, dz); rows outside the grid are empty
+        const uint32_t key0 = k - (q.x > 0 ? 1u : 0u), key1 = k + (q.x + 1 < c.ncell[0] ? 2u : 1u);
+        uint32_t rows_in = (q.y > 0 ? 1u : 0u) | 2u | (q.y + 1 < c.ncell[1] ? 4u : 0u);
+        if (DIM == 3) rows_in = (q.z > 0 ? rows_in : 0u) | rows_in << 3 | (q.z + 1 < c.ncell[2] ? rows_in << 6 : 0u);
+        if (!valid) rows_in = 0u;
+        auto range = [&](int r, uint32_t &b, uint32_t &e) {
+            b = e = 0u;
+            if (rows_in >> r & 1u) {
+                const uint32_t d = ((DIM == 3 ? r / 3 - 1 : 0) * (int)c.ncell[1] + r % 3 - 1) * (int)c.ncell[0];
+                b = ldro<NC>(w.cell_off + (key0 + d));
+                e = ldro<NC>(w.cell_off + (key1 + d));
+            }
+        };
+        constexpr uint32_t none = 0xffffffffu;
+        int row = 0;
+        uint32_t b, e, b1, e1;
+        range(0, b, e);
+        range(1, b1, e1);
+        uint32_t cb;              // first slot of the chunk to stage next (even)
+        float4 st0, st1;          // its slots 2 lane and 2 lane + 1
+        // the next chunk any lane needs, from `from` on in this row, else in
+        // the rows that follow
+        auto next_chunk = [&](uint32_t from) {
+            for (;;) {
+                const uint32_t lo = max(b, from);
+                cb = __reduce_min_sync(full, lo < e ? lo : none);
+                if (cb != none) break;
+                if (++row >= nrows) return;
+                b = b1;
+                e = e1;
+                range(row + 1, b1, e1);
+                from = 0u;
+            }
+            cb &= ~1u;
+            const uint32_t t = cb + 2u * lane;
+            st0 = ldro<NC>(w.spos + min(t, n - 1u));
+            st1 = ldro<NC>(w.spos + min(t + 1u, n - 1u));
+        };
+        next_chunk(0u);
+#pragma unroll 1
+        while (row < nrows) {
+            const uint32_t t = cb + 2u * lane;
+            __syncwarp();
+            sm.xy[lane] = make_float4(st0.x, st1.x, st0.y, st1.y);
+            sm.zs[lane] = make_uint4(__float_as_uint(st0.z), t | (st0.w == 1.0f ? 0u : kDensLevel2),
+                                     __float_as_uint(st1.z), (t + 1u) | (st1.w == 1.0f ? 0u : kDensLevel2));
+            __syncwarp();
+            // this lane's part of the chunk, then the next chunk's loads
+            const uint32_t lo = max(b, cb), hi = min(e, cb + 64u);
+            int left = lo < hi ? (int)(hi - lo) : 0;
+            uint32_t i = left ? lo - cb : 0u;
+            float thr0 = i & 1u ? -1.0f : reach2;
+            left += (int)(i & 1u);
+            i &= ~1u;
+            const bool own_row = row == own;
+            next_chunk(cb + 64u);
+            for (;;) {
+                if (own_row) {
+                    for (; left > 0 && at <= col_lim; i += 4, left -= 4, thr0 = reach2)
+                        quad(i, thr0, left, std::true_type());
+                } else {
+                    for (; left > 0 && at <= col_lim; i += 4, left -= 4, thr0 = reach2)
+                        quad(i, thr0, left, std::false_type());
+                }
+                const bool again = __any_sync(full, left > 0);   // a lane's buffer filled up
+                if (again || __any_sync(full, at > col_lim - FLUSH * 256u)) drain(false);
+                if (!again) break;
+            }
+        }
+        drain(true);
+        if (!valid) continue;
         rho = __fadd_rn(rho, c.mass[li] * poly6 * c.kernel6[li]);   // self term
         float r = rho / c.rest_density;
         const float gas = w.nscenes ? w.scene_tab[2 * min(w.sscene[s], w.nscenes - 1u) + 1].w : c.gas_constant;
@@ -507,19 +673,29 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
     }
 }
 
-template <int DIM, bool NC>
-__device__ __forceinline__ void density_body(const sph_config &c, Counters *cnt, const WorkPtrs &w)
+template <int DIM, int BS, bool NC, uint32_t CAP, uint32_t FLUSH>
+__device__ __forceinline__ void density_body(const sph_config &c, Counters *cnt, const WorkPtrs &w,
+                                             DensSmem<CAP> *smem)
 {
-    if (c.density_skip_r2 == 0.0f) density_walk<DIM, NC, false>(c, cnt, w);
-    else density_walk<DIM, NC, true>(c, cnt, w);
+    if (c.density_skip_r2 == 0.0f) density_walk<DIM, BS, NC, false, CAP, FLUSH>(c, cnt, w, smem);
+    else density_walk<DIM, BS, NC, true, CAP, FLUSH>(c, cnt, w, smem);
 }
 
 // The standalone kernel is instantiated per SKIP (the host picks it): one
-// walk per kernel keeps its registers at the walk's own need.
+// walk per kernel keeps its registers at the walk's own need.  24 buffer
+// entries per lane let seven 128-thread blocks reside (72 registers, 28 KB);
+// 20 entries drain more often (304 against 294 us on 1.24M particles), 28
+// leave less L1 (303).  Larger blocks take fewer entries to fit.
+template <int BS> constexpr uint32_t kDensCap = BS <= 128 ? 24 : 18;
+template <int BS> constexpr uint32_t kDensFlush = BS <= 128 ? 10 : 8;
+template <int BS> constexpr size_t kDensSmemBytes = sizeof(DensSmem<kDensCap<BS>>) * (BS / 32);
+
 template <int DIM, int BS = kThreads, bool SKIP = true>
 __global__ void __launch_bounds__(BS) k_density(sph_config c, Counters *__restrict__ cnt, WorkPtrs w)
 {
-    density_walk<DIM, true, SKIP>(c, cnt, w);
+    extern __shared__ __align__(16) unsigned char dens_smem[];
+    density_walk<DIM, BS, true, SKIP, kDensCap<BS>, kDensFlush<BS>>(
+        c, cnt, w, reinterpret_cast<DensSmem<kDensCap<BS>> *>(dens_smem));
 }
 
 // ------------------------------------------------------------ 6. force + integrate
@@ -550,11 +726,6 @@ __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counte
         const float ilap = c.lapc_poly6[li];
         const uint32_t sid = w.nscenes ? min(w.sscene[s], w.nscenes - 1u) : 0u;
         const float visc = w.nscenes ? w.scene_tab[2 * sid].w : c.viscosity;
-        const uint32_t k = w.skey[s];
-        uint3 q;
-        q.x = k % c.ncell[0];
-        q.y = (k / c.ncell[0]) % c.ncell[1];
-        q.z = DIM == 3 ? k / (c.ncell[0] * c.ncell[1]) : 0u;
         float fx = 0.f, fy = 0.f, fz = 0.f, gx = 0.f, gy = 0.f, gz = 0.f, lap = 0.f;
         if (DIM == 2)   // self term, SPH-2D/sph_system.cu:599-603 (0 with the integer 3/4)
             lap = __fmaf_rn(ilap * ai.w * hi2, __fsub_rn(0.0f, c.lapc_three_quarters * hi2), lap);
@@ -644,6 +815,7 @@ __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counte
                     if (accept_ab(a, b)) pair_ab(a, b);
                 }
         } else {
+            const uint3 q = cell_of_key<DIM>(c, w.skey[s]);
             warp_pairs<DIM, 0, NC>(c, w.cell_off, w.spos, valid, q, smem[wib], accept, pair);
         }
         if (!valid) continue;

@@ -185,13 +185,18 @@ __device__ __forceinline__ bool grid_scan(const PersistArgs &a, uint32_t &k, Cou
 // phase (scan_onepass_body): each block reads every count before its chunk.
 constexpr uint32_t kOnePassPerThread = 16;
 
+// The density buffer of a persistent warp: what fits beside its staged chunk
+// in the room the pair lists take.
+constexpr uint32_t kDensCapPersist = 16;
+static_assert(sizeof(DensSmem<kDensCapPersist>) <= sizeof(WarpPairSmem), "the union keeps its size");
+
 // One step's stages, from the hash (or, when the previous step hashed this
 // state already, from the cell scan) to the write-out.  Returns false, for
 // the whole block, once any block has given up at a barrier.
 template <int DIM, int BS>
 __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, Counters *cout, const CanonPtrs &in,
                                             const CanonPtrs &out, const WorkPtrs &w, const PersistArgs &a,
-                                            uint32_t &k, bool hashed, WarpPairSmem *pair, MergeSmem *merge)
+                                            uint32_t &k, bool hashed, WarpPairSmem *pair, MergeSmem *merge, DensSmem<kDensCapPersist> *dens)
 {
     if (!a.ranks && blockIdx.x == 0 && threadIdx.x == 0) {
         cin->n_split = 0u;
@@ -215,7 +220,7 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
     if (!grid_barrier(a, ++k, cin, cout)) return false;
     reorder_body<false>(cin, in, w);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    density_body<DIM, false>(c, cin, w);
+    density_body<DIM, BS, false, kDensCapPersist, 8>(c, cin, w, dens);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
     force_integrate_body<DIM, BS, false>(c, cin, w, pair);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
@@ -271,6 +276,7 @@ __global__ void __launch_bounds__(BS, 2) k_step_persistent(sph_config c, Counter
     __shared__ union {
         WarpPairSmem pair[BS / 32];
         MergeSmem merge[BS / 32];
+        DensSmem<kDensCapPersist> dens[BS / 32];
     } sm;
     const int p = a.parity;
     if (cnt[p].error & (1u << SPH_ERR_TIMEOUT)) {   // a step before gave up: nothing to step from
@@ -284,7 +290,8 @@ __global__ void __launch_bounds__(BS, 2) k_step_persistent(sph_config c, Counter
         Counters *cin = cnt + q, *cout = cnt + (q ^ 1);
         if (j > 0 && !grid_barrier(a, ++k, cin, cout)) return;
         const bool hashed = j > 0 || a.hash_ready != 0;
-        if (!step_stages<DIM, BS>(c, cin, cout, buf.b[q], buf.b[q ^ 1], w, a, k, hashed, sm.pair, sm.merge))
+        if (!step_stages<DIM, BS>(c, cin, cout, buf.b[q], buf.b[q ^ 1], w, a, k, hashed, sm.pair, sm.merge,
+                                  sm.dens))
             return;
     }
 }
