@@ -194,12 +194,15 @@ uint64_t launch_key(const sph_handle *h)
     }
 // SWITCH2 also sets the occupancy target M (minimum resident blocks per SM
 // handed to __launch_bounds__, i.e. the register budget the compiler works
-// to): 6 blocks of 128 / 3 of 256 (85 registers) by default, 8 / 4 (64
-// registers) for the register-capped build.
-#define SPH_BS_SWITCH2(bs, cap, ...)                                                    \
+// to): m128 blocks of 128 / 3 of 256 (85 registers) by default, 8 / 4 (64
+// registers) for the register-capped build.  Force takes m128 = 5: the 95
+// registers its four overlapping pairs use without spilling (six blocks spill
+// 56 bytes: 240 against 223 us on 1.24M adaptive particles, 153 against 147 on
+// 1.05M plain ones).  Energy takes 6 (80 registers, none spilled).
+#define SPH_BS_SWITCH2(bs, cap, m128, ...)                                              \
     switch ((bs) * 16 + ((cap) ? 1 : 0)) {                                              \
     case 128 * 16 + 1: { constexpr int B = 128, M = 8; __VA_ARGS__; } break;            \
-    case 128 * 16: { constexpr int B = 128, M = 6; __VA_ARGS__; } break;                \
+    case 128 * 16: { constexpr int B = 128, M = (m128); __VA_ARGS__; } break;           \
     case 256 * 16 + 1: { constexpr int B = 256, M = 4; __VA_ARGS__; } break;            \
     default: { constexpr int B = 256, M = 3; __VA_ARGS__; } break;                      \
     }
@@ -331,7 +334,7 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
         SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_DENSITY], launch_density<DIM, B, true>(h, gd, cin, w));
     }
     stage(h, "density");
-    SPH_BS_SWITCH2(h->tune_bs[SPH_TUNE_FORCE], h->tune_minb[SPH_TUNE_FORCE],
+    SPH_BS_SWITCH2(h->tune_bs[SPH_TUNE_FORCE], h->tune_minb[SPH_TUNE_FORCE], 5,
                    k_force_integrate<DIM, B, M><<<grid_st(h, nub, SPH_TUNE_FORCE), B, 0, s>>>(c, cin, w));
     stage(h, "force_integrate");
     // density grid + surface mid-step: stale cell lists, integrated positions
@@ -346,7 +349,7 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
         h->grid_valid = true;
         stage(h, "surface");
     }
-    SPH_BS_SWITCH2(h->tune_bs[SPH_TUNE_ENERGY], h->tune_minb[SPH_TUNE_ENERGY],
+    SPH_BS_SWITCH2(h->tune_bs[SPH_TUNE_ENERGY], h->tune_minb[SPH_TUNE_ENERGY], 6,
                    k_energy_split<DIM, B, M><<<grid_st(h, nub, SPH_TUNE_ENERGY), B, 0, s>>>(c, cin, in, w,
                                                                                           h->debug ? 1 : 0));
     stage(h, "energy_split");

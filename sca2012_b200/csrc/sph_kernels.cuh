@@ -207,6 +207,25 @@ __device__ __forceinline__ float r2_of(float4 a, float4 b, float &dx, float &dy,
     return t;
 }
 
+// 1/sqrt(x) as rsqrtf gives it, without the rescaling of denormal x (+inf
+// there, as for 0).
+__device__ __forceinline__ float rsqrt_normal(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// sqrt(x) from y = rsqrt_normal(x) by one Newton step with the residual in
+// one fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990): no branch
+// and no second special-function instruction.  Compared with __fsqrt_rn over
+// every FP32 value in [2.7e-20, 4e37]: the same bits.  Not for x = 0 (NaN).
+__device__ __forceinline__ float sqrt_of(float x, float y)
+{
+    const float g = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(0.5f, y), g);
+}
+
 __device__ __forceinline__ float split_score(const sph_config &c, float e, float s)
 {
     return __fmaf_rn(s, c.co_surface, __fmul_rn(e, c.co_energy));
@@ -703,6 +722,11 @@ __global__ void __launch_bounds__(BS) k_density(sph_config c, Counters *__restri
 // 2D SPH-2D/sph_system.cu:462-790), then the integrator and walls
 // (SPH-3D-2/sph_system.cu:204-322, SPH-2D/sph_system.cu:198-252).  The
 // integrated state goes to the *_n arrays so the loop never sees it.
+// Bound: the latency of the neighbour loads beside instruction issue (52 % of
+// the slots).  Pairs that branch on their tests and take the IEEE square root
+// (a branch and a second special-function instruction each) ran one after the
+// other; computed without branches, the terms of four pairs overlap.  1.24M
+// adaptive particles: 0.302 -> 0.223 ms; 1.05M plain: 0.193 -> 0.147 ms.
 template <int DIM, int BS, bool NC>
 __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counters *cnt, const WorkPtrs &w,
                                                      WarpPairSmem *smem)
@@ -737,65 +761,79 @@ __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counte
         const float jspk1 = c.kernel_h6_twice ? c.spiky[1] / c.kernel6[1] : c.spiky[1];
         const float jvis0 = c.kernel_h6_twice ? c.visco[0] / c.kernel6[0] : c.visco[0];
         const float jvis1 = c.kernel_h6_twice ? c.visco[1] / c.kernel6[1] : c.visco[1];
-        const float mimj0 = mi * c.mass[0], mimj1 = mi * c.mass[1];
+        const float hj0 = c.kernel[0], hj1 = c.kernel[1];
+        // lap enters the force only through surface_coef
+        const bool tension = c.surface_coef != 0.0f;
+        const float mm0 = mi * c.mass[0], mm1 = mi * c.mass[1], mms = li ? mm1 : mm0;
         auto accept = [&](uint32_t t, const float4 &pj) {
             float rx, ry, rz;
             const float r2 = r2_of<DIM>(pi, pj, rx, ry, rz);
             const float cut = pj.w == 1.0f ? cut0 : cut1;
             return t != s && r2 < cut && !(r2 < close);
         };
-        // pressure, viscosity and colour-field terms of one neighbour
-        // (a, b: the neighbour's two records)
-        auto pair_ab = [&](const float4 a, const float4 b) {
+        // Pressure, viscosity and colour-field terms of one neighbour (a, b: its
+        // two records), added when `in` and r^2 passes the pair test.  The terms
+        // are computed without a branch, so those of several pairs overlap in the
+        // pipeline; only the sums are conditional.  SAME: the neighbour's level is
+        // the particle's own, so the two kernels' terms are equal and half their
+        // sum is either one, exactly.
+        auto pair_ab = [&](bool in, const float4 a, const float4 b, auto SAME) {
             float rx, ry, rz;
             const float r2 = r2_of<DIM>(pi, a, rx, ry, rz);
-            const int lj = signbit(b.x) ? 1 : 0;
+            const bool lj = SAME.value ? li != 0 : signbit(b.x);
             const float mrj = fabsf(b.x);   // m_j/rho_j
-            const float r = __fsqrt_rn(r2);
-            float ipk = 0.f, ivk = 0.f, jpk = 0.f, jvk = 0.f;
+            const bool ok = in && r2 < (SAME.value ? hi2 : lj ? cut1 : cut0) && !(r2 < close);
+            const float ir = rsqrt_normal(r2), r = sqrt_of(r2, ir);
             const float ikr = __fsub_rn(hi, r);
-            if (ikr > 0.0f) {
-                ipk = ispk * ikr * ikr;
-                ivk = ivis * ikr;
-                const float x = hi2 - r2;
-                const float tg = igrad * mrj * x * x;   // -grad_poly6 * m_j/rho_j * (h^2-r^2)^2
-                gx = __fmaf_rn(tg, rx, gx); gy = __fmaf_rn(tg, ry, gy); gz = __fmaf_rn(tg, rz, gz);
+            const bool iin = ikr > 0.0f;
+            const float iq = iin ? ikr : 0.0f;
+            const float ipk = ispk * iq * iq, ivk = ivis * iq;
+            float pk = ipk, vk = ivk;   // half the two kernels' sums
+            if (!SAME.value) {
+                const float jkr = __fsub_rn(lj ? hj1 : hj0, r);
+                const float jq = jkr > 0.0f ? jkr : 0.0f;
+                pk = 0.5f * __fadd_rn(ipk, (lj ? jspk1 : jspk0) * jq * jq);
+                vk = 0.5f * __fadd_rn(ivk, (lj ? jvis1 : jvis0) * jq);
+            }
+            const float x = hi2 - r2;
+            const float tg = igrad * mrj * x * x;   // -grad_poly6 * m_j/rho_j * (h^2-r^2)^2
+            const float tp = (SAME.value ? mms : lj ? mm1 : mm0) * __fadd_rn(ai.z, a.w) * pk * ir;
+            const float tv = (ai.w * mrj) * visc * vk;
+            const float dvx = __fsub_rn(b.y, evi.x), dvy = __fsub_rn(b.z, evi.y),
+                        dvz = DIM == 3 ? __fsub_rn(b.w, evi.z) : 0.0f;
+            auto sums = [&](float sg, float sp, float sv) {
+                gx = __fmaf_rn(sg, rx, gx); gy = __fmaf_rn(sg, ry, gy);
+                if (DIM == 3) gz = __fmaf_rn(sg, rz, gz);
+                fx = __fmaf_rn(dvx, sv, __fmaf_rn(-rx, sp, fx));
+                fy = __fmaf_rn(dvy, sv, __fmaf_rn(-ry, sp, fy));
+                if (DIM == 3) fz = __fmaf_rn(dvz, sv, __fmaf_rn(-rz, sp, fz));
+            };
+            if (tension && ok && iin)
                 lap = __fmaf_rn(ilap * mrj * x, __fsub_rn(r2, c.lapc_three_quarters * x), lap);
+            if (SAME.value) {
+                if (ok) sums(iin ? tg : 0.0f, tp, tv);
+            } else {   // a zero term leaves a sum as it is
+                sums(ok && iin ? tg : 0.0f, ok ? tp : 0.0f, ok ? tv : 0.0f);
             }
-            const float jkr = __fsub_rn(c.kernel[lj], r);
-            if (jkr > 0.0f) {
-                jpk = (lj ? jspk1 : jspk0) * jkr * jkr;
-                jvk = (lj ? jvis1 : jvis0) * jkr;
-            }
-            // 1/r from the approximate reciprocal square root of r^2 (the h - r
-            // decisions above keep the IEEE square root)
-            const float tp = (lj ? mimj1 : mimj0) * __fadd_rn(ai.z, a.w) * __fadd_rn(ipk, jpk) * 0.5f * rsqrtf(r2);
-            const float tv = (ai.w * mrj) * visc * __fadd_rn(ivk, jvk) * 0.5f;
-            fx = __fmaf_rn(__fsub_rn(b.y, evi.x), tv, __fmaf_rn(-rx, tp, fx));
-            fy = __fmaf_rn(__fsub_rn(b.z, evi.y), tv, __fmaf_rn(-ry, tp, fy));
-            if (DIM == 3) fz = __fmaf_rn(__fsub_rn(b.w, evi.z), tv, __fmaf_rn(-rz, tp, fz));
         };
-        // the walk's test for a list entry (a list never holds the particle itself)
-        auto accept_ab = [&](const float4 &a, const float4 &b) {
-            float rx, ry, rz;
-            const float r2 = r2_of<DIM>(pi, a, rx, ry, rz);
-            const float cut = signbit(b.x) ? cut1 : cut0;
-            return r2 < cut && !(r2 < close);
-        };
-        auto pair = [&](uint32_t t) { pair_ab(w.fnb_a[t], w.fnb_b[t]); };
+        auto pair = [&](uint32_t t) { pair_ab(true, w.fnb_a[t], w.fnb_b[t], std::false_type()); };
         const unsigned full = 0xffffffffu;
         const uint32_t nf = valid && w.nlist ? w.ncnt[s] : 0u;
         if (__all_sync(full, w.nlist != nullptr && nf <= kNbrListCap)) {
             // the density pass's candidates, filtered by the walk's test: same
             // neighbours, same order as the walk
             const uint32_t m = __reduce_max_sync(full, nf);
-            uint32_t kk = 0;
-            // four entries per 16-byte load, their neighbours' loads issued
-            // before the math (entries past nf are replaced by the particle itself)
-            if (4 < m) prefetch_l2(w.nlist + nl_at(w, s, 4));
-            for (; kk + 4 <= m; kk += 4) {
-                if (kk + 8 < m) prefetch_l2(w.nlist + nl_at(w, s, kk + 8));   // 2 rounds ahead
-                const uint4 t4 = *reinterpret_cast<const uint4 *>(w.nlist + nl_at(w, s, kk));
+            // four entries per 16-byte load, a round ahead of their use; the
+            // neighbours' loads issued before the math (entries past nf are
+            // replaced by the particle itself)
+            const uint4 *lp = reinterpret_cast<const uint4 *>(w.nlist) + s;   // chunk j at lp[j * nl_stride]
+            uint4 nxt = m ? *lp : make_uint4(s, s, s, s);
+            if (4 < m) prefetch_l2(lp + w.nl_stride);
+            for (uint32_t kk = 0; kk < m; kk += 4) {
+                const uint4 t4 = nxt;
+                lp += w.nl_stride;
+                if (kk + 8 < m) prefetch_l2(lp + w.nl_stride);   // 2 rounds ahead
+                if (kk + 4 < m) nxt = *lp;
                 const uint32_t tt[4] = {kk < nf ? t4.x : s, kk + 1 < nf ? t4.y : s, kk + 2 < nf ? t4.z : s,
                                         kk + 3 < nf ? t4.w : s};
                 float4 na[4], nb[4];
@@ -804,16 +842,18 @@ __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counte
                     na[u] = w.fnb_a[tt[u]];
                     nb[u] = w.fnb_b[tt[u]];
                 }
+                // one level among the warp's pairs (most of the fluid): the shorter terms
+                const uint32_t own = li ? 0x80000000u : 0u;
+                const uint32_t other = (__float_as_uint(nb[0].x) ^ own) | (__float_as_uint(nb[1].x) ^ own) |
+                                       (__float_as_uint(nb[2].x) ^ own) | (__float_as_uint(nb[3].x) ^ own);
+                if (__any_sync(full, (int)other < 0)) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (kk + u < nf && accept_ab(na[u], nb[u])) pair_ab(na[u], nb[u]);
-            }
-            for (; kk < m; ++kk)
-                if (kk < nf) {
-                    const uint32_t t = w.nlist[nl_at(w, s, kk)];
-                    const float4 a = w.fnb_a[t], b = w.fnb_b[t];
-                    if (accept_ab(a, b)) pair_ab(a, b);
+                    for (int u = 0; u < 4; ++u) pair_ab(kk + u < nf, na[u], nb[u], std::false_type());
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) pair_ab(kk + u < nf, na[u], nb[u], std::true_type());
                 }
+            }
         } else {
             const uint3 q = cell_of_key<DIM>(c, w.skey[s]);
             warp_pairs<DIM, 0, NC>(c, w.cell_off, w.spos, valid, q, smem[wib], accept, pair);

@@ -188,7 +188,6 @@ constexpr uint32_t kOnePassPerThread = 16;
 // The density buffer of a persistent warp: what fits beside its staged chunk
 // in the room the pair lists take.
 constexpr uint32_t kDensCapPersist = 16;
-static_assert(sizeof(DensSmem<kDensCapPersist>) <= sizeof(WarpPairSmem), "the union keeps its size");
 
 // One step's stages, from the hash (or, when the previous step hashed this
 // state already, from the cell scan) to the write-out.  Returns false, for
