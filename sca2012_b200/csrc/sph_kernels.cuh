@@ -359,7 +359,12 @@ __global__ void __launch_bounds__(BS) k_reorder(const Counters *__restrict__ cnt
 // order.  Flushing together keeps the expensive pair math converged (lists
 // fill at similar rates, so few lanes idle in a round), and every particle's
 // sums take the same order whichever particles share its warp.
-constexpr uint32_t kWarpCap = 40;             // list fill that triggers a warp flush (44 x 32 x 4 B per warp)
+// List fill that triggers a warp flush (24 x 32 x 4 B per warp).  The lists
+// take shared memory from the L1 that serves the neighbour loads of the warps
+// that read candidate lists: 40 entries held the L1 to 60-67 % hits there
+// (energy 251 us on 1.24M particles), 20 allow 69-71 % (246); a pass that
+// walks every stencil loses what 40 gained (2 %).
+constexpr uint32_t kWarpCap = 20;
 constexpr uint32_t kWarpSlot = kWarpCap + 4;  // a step can add 4 more before the check
 
 struct NbrPV { float4 p, v; };       // position, velocity
@@ -988,11 +993,36 @@ __global__ void __launch_bounds__(BS, MINB) k_force_integrate(sph_config c, Coun
 // Wavelet energy on the STALE cell lists (built at step start) with the NEW
 // positions (SPH-3D-2/sph_system.cu:1169-1546), then the split decision
 // (decide_adaptive_kernel, :1548-1574) written per particle index.
+// Bound: the L1 cost of gathering 32 bytes per list entry (73 % of its data
+// pipe; the gathers alone take 0.85 of the kernel's time).  The pair terms, x
+// and y as packed FP32 and without branches, take 32M instead of 50M
+// instructions on 387,000 particles.  1.24M adaptive particles: 0.252 ->
+// 0.215 ms; 1.05M plain: 0.151 -> 0.134 ms.
+// psi(x) = amp * (x^2/4 - 1) * EXP^(-x^2/8), EXP = 2.718281f (sigma = 2), for
+// |x| < 30: x^2/4 is exact, so one fused multiply-add rounds as the difference
+// does; the exponent's factor 1/8 is an exact scaling; and the exponential is
+// exp2f's without its rescaling of results below 2^-126.
+__device__ __forceinline__ float ex2_normal(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 __device__ __forceinline__ float wavelet(float x, float amp)
 {
-    // psi(x) = amp * (x^2/4 - 1) * EXP^(-x^2/8), EXP = 2.718281f (sigma = 2)
-    const float x2 = x * x;
-    return amp * __fsub_rn(x2 * 0.25f, 1.0f) * exp2f(-x2 * 0.125f * 1.44269476f);
+    const float x2 = __fmul_rn(x, x);
+    return __fmul_rn(__fmul_rn(amp, __fmaf_rn(x2, 0.25f, -1.0f)), ex2_normal(__fmul_rn(x2, -0.125f * 1.44269476f)));
+}
+
+// Two components at once (each half rounds as wavelet does).
+__device__ __forceinline__ float2 wavelet2(float2 x, float amp)
+{
+    const float2 x2 = __fmul2_rn(x, x);
+    const float2 e = __fmul2_rn(x2, make_float2(-0.125f * 1.44269476f, -0.125f * 1.44269476f));
+    return __fmul2_rn(__fmul2_rn(make_float2(amp, amp), __ffma2_rn(x2, make_float2(0.25f, 0.25f),
+                                                                   make_float2(-1.0f, -1.0f))),
+                      make_float2(ex2_normal(e.x), ex2_normal(e.y)));
 }
 
 template <int DIM, int BS, bool NC>
@@ -1016,7 +1046,8 @@ __device__ __forceinline__ void energy_split_body(const sph_config &c, Counters 
         const float h = c.kernel[lk], h2 = c.kernel2[lk];
         const float ih = 1.0f / h, isq = 1.0f / sqrtf(h);
         const uint3 q = cell_of<DIM>(c, pi);
-        float tsx = 0.f, tsy = 0.f, tsz = 0.f, tvx = 0.f, tvy = 0.f, tvz = 0.f;
+        float2 ts = make_float2(0.f, 0.f), tv = ts;   // x and y sums, z below
+        float tsz = 0.f, tvz = 0.f;
         const float skip = c.energy_skip_close ? c.close_r2 : 0.0f;   // :1229-1232 (2D keeps close pairs)
         // j != i with skip <= r^2 < h^2 (:1222-1233), on the stale lists
         auto accept = [&](uint32_t t, const float4 &pj) {
@@ -1024,20 +1055,32 @@ __device__ __forceinline__ void energy_split_body(const sph_config &c, Counters 
             const float r2 = r2_of<DIM>(pi, pj, rx, ry, rz);
             return t != s && r2 < h2 && !(r2 < skip);
         };
-        // the wavelet transform of one neighbour (its loads fetched ahead)
+        // the wavelet transform of one neighbour (its loads fetched ahead);
+        // x and y as packed FP32, each half rounded as alone
         auto fetch = [&](uint32_t t) { return NbrPV{w.spos_n[t], w.svel_n[t]}; };
-        auto use = [&](const NbrPV &g) {
-            const float4 pj = g.p, vj = g.v;
-            float rx, ry, rz;
-            r2_of<DIM>(pi, pj, rx, ry, rz);
-            const float wx = wavelet(rx * ih, amp), wy = wavelet(ry * ih, amp);
-            tsx = __fadd_rn(tsx, wx); tsy = __fadd_rn(tsy, wy);
-            tvx = __fmaf_rn(vj.x * wx, isq, tvx); tvy = __fmaf_rn(vj.y * wy, isq, tvy);
-            if (DIM == 3) {
-                const float wz = wavelet(rz * ih, amp);
-                tsz = __fadd_rn(tsz, wz);
-                tvz = __fmaf_rn(vj.z * wz, isq, tvz);
+        auto add = [&](bool ok, const NbrPV &g, float2 rxy, float rz) {
+            const float2 wxy = wavelet2(__fmul2_rn(rxy, make_float2(ih, ih)), amp);
+            const float2 pxy = __fmul2_rn(make_float2(g.v.x, g.v.y), wxy);
+            const float wz = DIM == 3 ? wavelet(__fmul_rn(rz, ih), amp) : 0.0f, pz = __fmul_rn(g.v.z, wz);
+            if (ok) {
+                ts = __fadd2_rn(ts, wxy);
+                tv = __ffma2_rn(pxy, make_float2(isq, isq), tv);
+                if (DIM == 3) {
+                    tsz = __fadd_rn(tsz, wz);
+                    tvz = __fmaf_rn(pz, isq, tvz);
+                }
             }
+        };
+        auto use = [&](const NbrPV &g) {
+            float rx, ry, rz;
+            r2_of<DIM>(pi, g.p, rx, ry, rz);
+            add(true, g, make_float2(rx, ry), rz);
+        };
+        // a list entry: the walk's test (a list never holds the particle itself)
+        auto use_listed = [&](bool in, const NbrPV &g) {
+            float rx, ry, rz;
+            const float r2 = r2_of<DIM>(pi, g.p, rx, ry, rz);
+            add(in && r2 < h2 && !(r2 < skip), g, make_float2(rx, ry), rz);
         };
         // the density pass's candidates when the particle kept its cell and the
         // step's moves fit the margin; the stencil walk otherwise
@@ -1055,13 +1098,17 @@ __device__ __forceinline__ void energy_split_body(const sph_config &c, Counters 
         }
         const uint32_t m = __reduce_max_sync(0xffffffffu, ne);
         if (m) {
-            // four entries per 16-byte load, their neighbours fetched before the
-            // math (entries past ne are replaced by the particle itself)
-            if (4 < m) prefetch_l2(w.nlist + nl_at(w, s, 4));
+            // four entries per 16-byte load, a round ahead of their use; their
+            // neighbours fetched before the math (entries past ne are replaced
+            // by the particle itself)
+            const uint4 *lp = reinterpret_cast<const uint4 *>(w.nlist) + s;   // chunk j at lp[j * nl_stride]
+            uint4 nxt = ne ? *lp : make_uint4(s, s, s, s);
+            if (4 < m) prefetch_l2(lp + w.nl_stride);
             for (uint32_t kk = 0; kk < m; kk += 4) {
-                if (kk + 8 < m) prefetch_l2(w.nlist + nl_at(w, s, kk + 8));   // 2 rounds ahead
-                const uint4 t4 = kk < ne ? *reinterpret_cast<const uint4 *>(w.nlist + nl_at(w, s, kk))
-                                         : make_uint4(s, s, s, s);
+                const uint4 t4 = nxt;
+                lp += w.nl_stride;
+                if (kk + 8 < m) prefetch_l2(lp + w.nl_stride);   // 2 rounds ahead
+                if (kk + 4 < ne) nxt = *lp;
                 const uint32_t tt[4] = {kk < ne ? t4.x : s, kk + 1 < ne ? t4.y : s, kk + 2 < ne ? t4.z : s,
                                         kk + 3 < ne ? t4.w : s};
                 NbrPV g[4];
@@ -1069,12 +1116,13 @@ __device__ __forceinline__ void energy_split_body(const sph_config &c, Counters 
                 for (int u = 0; u < 4; ++u) g[u] = fetch(tt[u]);
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    if (kk + u < ne && accept(tt[u], g[u].p)) use(g[u]);
+                    use_listed(kk + u < ne, g[u]);
             }
         }
         warp_pairs<DIM, 4, NC>(c, w.cell_off, w.spos_n, walk, q, smem[wib], accept, fetch_use(fetch, use), s);
         if (!valid) continue;
-        tvx /= tsx; tvy /= tsy; tvz = DIM == 3 ? tvz / tsz : 0.f;
+        const float tvx = tv.x / ts.x, tvy = tv.y / ts.y;
+        tvz = DIM == 3 ? tvz / tsz : 0.f;
         float energy = 0.5f * __fmaf_rn(tvx, tvx, __fmul_rn(tvy, tvy));
         if (c.energy_mass_weight) energy *= c.mass[li];
         w.senergy[s] = energy;
