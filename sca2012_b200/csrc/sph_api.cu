@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -39,6 +40,7 @@ struct sph_handle {
     WorkPtrs w;
     uint32_t *scan_blocks = nullptr;  // kScanBlocks * 2 u32
     uint32_t *scan_grand = nullptr;   // scratch total
+    int scan_cluster = 0;             // blocks of a one-cluster scan (0: two launches)
     uint32_t *stat_buf = nullptr;     // sph_last_step_stats: level-2 count
     uint32_t n_ub = 0;                // host upper bound of the live count
     uint32_t n_last_sorted = 0;       // count the last step started with (host copy)
@@ -207,17 +209,92 @@ uint64_t launch_key(const sph_handle *h)
     default: { constexpr int B = 256, M = 3; __VA_ARGS__; } break;                      \
     }
 
-// Exclusive scan of u32 `in` -> `out`; length from len_ptr (device) or
-// len_const.  skip_if_zero: a device count of the nonzero inputs (0: the
-// output is all zeros and is written without a scan).
-void scan_u32(sph_handle *h, const uint32_t *in, uint32_t *out, const uint32_t *len_ptr, uint32_t len_const,
-              uint32_t *grand, int total_at_len, uint32_t *list, const uint32_t *skip_if_zero = nullptr)
+// Whether a scan of at most `bound` elements runs as one cluster.  16 SMs cost
+// less than the second launch (and, for the cell counts, the memset) of a full
+// grid up to about 800,000 elements: cell scan 11.0 against 15.2 us at 262,144
+// cells, 21.5 against 19.2 at 1,048,576, 59 against 34 at 4M.  A rank scan
+// whose flags may be all zero (most steps) only checks their count then, 6
+// against 11-13 us, which pays up to a bound of 4M (the host's bound of the
+// particle count, up to four times the count itself).
+constexpr uint32_t kClusterScanMax = 3u << 18, kClusterRankMax = 1u << 22;
+
+bool scan_as_cluster(const sph_handle *h, uint32_t bound, bool ranks)
 {
-    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, len_ptr, len_const, h->scan_blocks,
+    return h->scan_cluster > 0 && bound <= (ranks ? kClusterRankMax : kClusterScanMax);
+}
+
+template <class... P, class... A>
+void launch_cluster(sph_handle *h, void (*kern)(P...), A... args)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(h->scan_cluster);
+    lc.blockDim = dim3(kClusterScanThreads);
+    lc.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = h->scan_cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    cudaLaunchKernelEx(&lc, kern, P(args)...);
+    h->last_launches += 1;
+}
+
+// Cluster size of the one-launch scans on a device: 16 blocks, else 8, else
+// none (0).  A property of the device, asked once per process (the occupancy
+// query takes about a millisecond).
+int query_scan_cluster(int device)
+{
+    constexpr int kMaxDevices = 64;
+    static std::atomic<int> known[kMaxDevices];   // size + 1; 0: not asked yet
+    if (device >= 0 && device < kMaxDevices) {
+        if (const int k = known[device].load()) return k - 1;
+        const int size = query_scan_cluster(-1);
+        known[device].store(size + 1);
+        return size;
+    }
+    for (int size : {kClusterScanBlocks, 8}) {
+        bool ok = true;
+        for (const void *kern : {(const void *)k_scan_cluster, (const void *)k_split_ranks}) {
+            if (size > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                ok = false;
+            cudaLaunchConfig_t lc = {};
+            lc.gridDim = dim3(size);
+            lc.blockDim = dim3(kClusterScanThreads);
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = size;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            lc.attrs = attr;
+            lc.numAttrs = 1;
+            int n = 0;
+            ok = ok && cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess && n >= 1;
+        }
+        cudaGetLastError();
+        if (ok) return size;
+    }
+    return 0;
+}
+
+// Exclusive scan of u32 `in` -> `out`; length from len_ptr (device, at most
+// `bound`) or bound itself.  skip_if_zero: a device count of the nonzero
+// inputs (0: only the total is written).  clear: zero the input behind the scan.
+void scan_u32(sph_handle *h, uint32_t *in, uint32_t *out, const uint32_t *len_ptr, uint32_t bound, uint32_t *grand,
+              int total_at_len, uint32_t *list, const uint32_t *skip_if_zero = nullptr, bool clear = false)
+{
+    if (scan_as_cluster(h, bound, skip_if_zero != nullptr)) {
+        launch_cluster(h, k_scan_cluster, ClusterScan{in, out, len_ptr, bound, grand, list, skip_if_zero, total_at_len,
+                                                      clear ? 1 : 0});
+        return;
+    }
+    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, len_ptr, bound, h->scan_blocks,
                                                                        skip_if_zero);
-    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, len_ptr, len_const, h->scan_blocks,
+    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, len_ptr, bound, h->scan_blocks,
                                                                         grand, total_at_len, list, skip_if_zero);
     h->last_launches += 2;
+    if (clear) cudaMemsetAsync(in, 0, sizeof(uint32_t) * bound, h->stream);
 }
 
 // Marching cubes over the current device grid: classify, scan, emit.
@@ -317,9 +394,8 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
         hash_prologue<DIM>(h);
         stage(h, "hash");
     }
-    scan_u32(h, w.cell_count, w.cell_off, nullptr, h->ncells, h->scan_grand, 1, nullptr);
-    // the scan has read the counts: cleared for the write-out's hash of the next state
-    cudaMemsetAsync(w.cell_count, 0, sizeof(uint32_t) * h->ncells, s);
+    // the counts are cleared behind the scan, for the write-out's hash of the next state
+    scan_u32(h, w.cell_count, w.cell_off, nullptr, h->ncells, h->scan_grand, 1, nullptr, nullptr, true);
     h->counts_zero = false;
     stage(h, "scan_cells");
     SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_SCATTER], k_scatter<B><<<grid_st(h, nub, SPH_TUNE_SCATTER), B, 0, s>>>(cin, w));
@@ -353,20 +429,27 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
                    k_energy_split<DIM, B, M><<<grid_st(h, nub, SPH_TUNE_ENERGY), B, 0, s>>>(c, cin, in, w,
                                                                                           h->debug ? 1 : 0));
     stage(h, "energy_split");
-    h->last_launches += 6;
-    scan_u32(h, w.split_c, w.split_rank, &cin->n, 0, &cin->n_split, 0, w.split_list, &cin->split_flags);
-    k_split_guard<<<1, 1, 0, s>>>(c, cin, h->cap);
-    h->last_launches += 1;
-    stage(h, "scan_split");
+    h->last_launches += 5;
+    if (c.use_split) {   // else no particle is flagged
+        if (scan_as_cluster(h, nub, true)) {
+            launch_cluster(h, k_split_ranks, ClusterScan{w.split_c, w.split_rank, &cin->n, nub, nullptr, w.split_list,
+                                                         nullptr, 0, 0}, c, cin, h->cap);
+        } else {
+            scan_u32(h, w.split_c, w.split_rank, &cin->n, nub, &cin->n_split, 0, w.split_list, &cin->split_flags);
+            k_split_guard<<<1, 1, 0, s>>>(c, cin, h->cap);
+            h->last_launches += 1;
+        }
+        stage(h, "scan_split");
+    }
     if (c.use_merge) {   // one lane per cell, a warp scans 32 cells at a time
         SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_MERGE],
                       k_merge<DIM, B><<<grid_st(h, h->ncells, SPH_TUNE_MERGE), B, 0, s>>>(c, cin, in, w, h->ncells,
                                                                                           h->cap));
         h->last_launches += 1;
         stage(h, "merge");
+        scan_u32(h, w.removed_c, w.removed_rank, &cin->n, nub, &cin->n_removed, 0, nullptr, &cin->removed_flags);
+        stage(h, "scan_removed");
     }
-    scan_u32(h, w.removed_c, w.removed_rank, &cin->n, 0, &cin->n_removed, 0, nullptr, &cin->removed_flags);
-    stage(h, "scan_removed");
     SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_WRITE],
                   k_write<DIM, B><<<grid_st(h, nub, SPH_TUNE_WRITE), B, 0, s>>>(c, cin, cout, in, out, w, 1));
     h->last_launches += 1;
@@ -603,6 +686,7 @@ int sph_create(const sph_config *cfg, sph_handle **out)
         return SPH_ERR_CUDA;
     }
     h->own_stream = h->stream;
+    h->scan_cluster = query_scan_cluster(h->device);
     h->cap = cfg->max_particle;
     h->ncells = total_cells(*cfg);
     const size_t cap = h->cap, C = h->ncells;

@@ -31,6 +31,7 @@
 #include <cstdint>
 #include <type_traits>
 #include "../../include/sph/sph.h"
+#include "sph_scan.cuh"
 
 namespace sph {
 
@@ -47,7 +48,7 @@ struct Counters {
     uint32_t disp2_max;    // bits of the step's largest squared displacement (FP32 >= 0), by the force pass
     uint32_t split_flags;  // particles the energy pass flagged to split this step
     uint32_t removed_flags;  // particles the merge pass flagged as merged away this step
-                           // (a rank scan whose flags are all zero writes zeros instead of scanning)
+                           // (at 0 the ranks of a kind are not written: every reader tests the count)
     uint32_t merge_candidates;  // particles that may be merge-eligible this step, by the energy
                            // pass (at 0 the merge pass has nothing to do and returns at once)
 };
@@ -489,7 +490,10 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
     const unsigned full = 0xffffffffu;
     const uint32_t n = cnt->n;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) cnt->disp2_max = 0u;   // the force pass takes the max
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        cnt->disp2_max = 0u;   // the force pass takes the max
+        cnt->n_split = cnt->n_removed = cnt->split_off = 0u;   // set by the rank scans a step runs
+    }
     DensSmem<CAP> &sm = smem[wib];
     uint2 *const col = &sm.ent[0][lane];
     // the append position as a shared-memory address (256 bytes per entry)
@@ -1174,10 +1178,10 @@ __global__ void __launch_bounds__(BS, MINB) k_energy_split(sph_config c, Counter
 // Capacity guard after the split scan: if the children would not fit, this
 // step runs without splits and reports SPH_ERR_CAPACITY (the reference writes
 // past its buffer, SPH-3D-2/sph_system.cu:1645-1656).
-__device__ __forceinline__ void split_guard_body(const sph_config &c, Counters *cnt, uint32_t cap)
+__device__ __forceinline__ void split_guard_body(const sph_config &c, Counters *cnt, uint32_t n_split, uint32_t cap)
 {
     uint64_t extra = c.split_ways == 4 ? 3u : 1u;
-    uint64_t after = (uint64_t)cnt->n + (uint64_t)cnt->n_split * extra;
+    uint64_t after = (uint64_t)cnt->n + (uint64_t)n_split * extra;
     if (after > cap) {
         cnt->split_off = 1u;
         cnt->error |= 1u << SPH_ERR_CAPACITY;
@@ -1186,7 +1190,30 @@ __device__ __forceinline__ void split_guard_body(const sph_config &c, Counters *
     }
 }
 
-__global__ void k_split_guard(const sph_config c, Counters *cnt, uint32_t cap) { split_guard_body(c, cnt, cap); }
+__global__ void k_split_guard(const sph_config c, Counters *cnt, uint32_t cap)
+{
+    split_guard_body(c, cnt, cnt->n_split, cap);
+}
+
+__global__ void __launch_bounds__(kClusterScanThreads) k_scan_cluster(ClusterScan j)
+{
+    if (j.skip_if_zero && *j.skip_if_zero == 0u) {
+        if (blockIdx.x == 0 && threadIdx.x == 0 && j.grand) *j.grand = 0u;
+        return;
+    }
+    cluster_scan_body(j);
+}
+
+// The split rank scan as one cluster, with the guard on its total.
+__global__ void __launch_bounds__(kClusterScanThreads) k_split_ranks(ClusterScan j, const sph_config c, Counters *cnt,
+                                                                    uint32_t cap)
+{
+    const uint32_t total = cnt->split_flags ? cluster_scan_body(j) : 0u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        cnt->n_split = total;
+        split_guard_body(c, cnt, total, cap);
+    }
+}
 
 // ------------------------------------------------------------ 8. merge
 // One warp per cell over its sorted members (merge_kernel,
@@ -1429,8 +1456,8 @@ __global__ void __launch_bounds__(BS) k_merge(sph_config c, Counters *__restrict
 // [surviving particles in index order][children in split order][removed].
 // Children follow adaptive_particle_kernel (:1576-1615; 3D-4 :1583-1656;
 // 2D :1133-1160).  Writes the other canonical buffer.
-// ranks = false: the step ran no split and removal scans (split and merge
-// both off), so there are no children and nothing is removed.
+// The split and removal ranks (and the flags behind them) are read only where
+// the step's counts of them are not zero.
 // hash_next: also hash every particle it writes for the next step (hash_one
 // at its new index; the cell counts were cleared after this step's scan), so
 // the next step starts at the cell scan.
@@ -1440,14 +1467,15 @@ __global__ void __launch_bounds__(BS) k_merge(sph_config c, Counters *__restrict
 template <int DIM>
 __device__ __forceinline__ void write_body(const sph_config &c, const Counters *cnt, Counters *cnt_next,
                                            const CanonPtrs &in, const CanonPtrs &out, const WorkPtrs &w,
-                                           bool ranks = true, bool hash_next = false)
+                                           bool hash_next = false)
 {
     const uint32_t n = cnt->n;
-    const uint32_t split_on = ranks && !cnt->split_off ? 1u : 0u;
+    const bool split_on = cnt->split_flags != 0u && !cnt->split_off;
+    const bool merged = cnt->removed_flags != 0u;
     const uint32_t ways = c.split_ways == 4 ? 4u : 2u;
     const uint32_t extra = ways - 1u;
     const uint32_t n_split = split_on ? cnt->n_split : 0u;
-    const uint32_t n_removed = ranks ? cnt->n_removed : 0u;
+    const uint32_t n_removed = merged ? cnt->n_removed : 0u;
     const uint32_t n_after = n + n_split * extra;
     const uint32_t n_live = n_after - n_removed;
     const float hs2 = c.kernel[1] / 2.0f;
@@ -1465,9 +1493,9 @@ __device__ __forceinline__ void write_body(const sph_config &c, const Counters *
     // writes (survivors keep their order) stay coalesced
     for (uint32_t i = grid_stride_start(); i < n; i += grid_stride()) {
         const uint32_t s = w.inv[i];
-        const uint32_t sp = split_on & w.split_c[i];
-        const uint32_t rm = ranks ? w.removed_c[i] : 0u;
-        const uint32_t rr = ranks ? w.removed_rank[i] : 0u;
+        const uint32_t sp = split_on ? w.split_c[i] : 0u;
+        const uint32_t rm = merged ? w.removed_c[i] : 0u;
+        const uint32_t rr = merged ? w.removed_rank[i] : 0u;
         const uint32_t dst = rm ? n_live + rr : i - rr;
         float4 p = w.spos_n[s], v = w.svel_n[s], e = w.sev_n[s];
         uint32_t inter = (c.merge_rule == SPH_MERGE_INTERIOR || c.merge_rule == SPH_MERGE_SIBLING) ? w.sinter[s] : 0u;
@@ -1480,12 +1508,12 @@ __device__ __forceinline__ void write_body(const sph_config &c, const Counters *
         float4 plo = w.pos_comp ? w.spos_lo_n[s] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float4 plo_pre = plo;
         uint32_t sib = kEmpty;
-        if (!rm && !w.leader[s]) {
+        const uint32_t leader = merged ? w.leader[s] : 0u;
+        if (!rm && !leader) {
             const uint32_t j = in.sibling[i];
-            if (j < n) sib = j - (ranks ? w.removed_rank[j] : 0u);
+            if (j < n) sib = j - (merged ? w.removed_rank[j] : 0u);
         }
         if (sp) sib = n - n_removed + w.split_rank[i] * extra;   // the first child
-        const uint32_t leader = w.leader[s];
         if (leader) {
             plo = make_float4(0.f, 0.f, 0.f, 0.f);   // a merged position is a fresh FP32 mean
             p = w.mpos[s]; v = w.mvel[s]; e = w.mev[s];
@@ -1572,7 +1600,7 @@ __global__ void __launch_bounds__(BS) k_write(sph_config c, const Counters *__re
                                                    Counters *__restrict__ cnt_next, CanonPtrs in, CanonPtrs out,
                                                    WorkPtrs w, int hash_next)
 {
-    write_body<DIM>(c, cnt, cnt_next, in, out, w, true, hash_next != 0);
+    write_body<DIM>(c, cnt, cnt_next, in, out, w, hash_next != 0);
 }
 
 // ------------------------------------------------------------ reference-layout records

@@ -2,8 +2,8 @@
 //
 // The reference launches every stage of a step separately
 // (SPHSystem::animation, SPH-3D-2/sph_system.cpp:302-404; animate,
-// SPH-2D/sph_system.cpp:190-264), and so does sph_step's ordinary path (13
-// launches and a memset, or one replayed CUDA graph of them).  On small scenes the step
+// SPH-2D/sph_system.cpp:190-264), and so does sph_step's ordinary path (7
+// launches, 10 with split and merge, or one replayed CUDA graph of them).  On small scenes the step
 // is then bound by the launches and the drain between them, not by the work.
 // k_step_persistent runs the same stage bodies (sph_kernels.cuh,
 // sph_scan.cuh) in one launch whose blocks are all resident (a cooperative
@@ -17,7 +17,7 @@
 // (the bracketed stages only when split or merge is on).  The write-out also
 // hashes the state it writes for the next step, so a step whose state was
 // written by a step before starts at the cell scan: 12 barriers per step with
-// adaptivity.  Without it the write-out runs in the energy stage
+// adaptivity (7 when nothing splits or merges).  Without it the write-out runs in the energy stage
 // (write_hash_by_slot_body), and a small cell grid is scanned in one phase:
 // 5 barriers per step.  One launch runs several steps without splits, one
 // more barrier between two of them.  Each scan's second phase has every block sum
@@ -197,11 +197,6 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
                                             const CanonPtrs &out, const WorkPtrs &w, const PersistArgs &a,
                                             uint32_t &k, bool hashed, WarpPairSmem *pair, MergeSmem *merge, DensSmem<kDensCapPersist> *dens)
 {
-    if (!a.ranks && blockIdx.x == 0 && threadIdx.x == 0) {
-        cin->n_split = 0u;
-        cin->n_removed = 0u;
-        cin->split_off = 0u;
-    }
     if (!hashed) {
         hash_body<DIM>(c, cin, in, w);
         if (!grid_barrier(a, ++k, cin, cout)) return false;
@@ -230,16 +225,13 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
     }
     if (!grid_barrier(a, ++k, cin, cout)) return false;
     const uint32_t n = cin->n;
-    // a scan of all-zero flags is all zeros: written directly, no barrier
+    // with no flags there are no ranks, and nothing to guard
     if (cin->split_flags) {
         if (!grid_scan<uint32_t>(a, k, cin, cout, w.split_c, w.split_rank, n, &cin->n_split, 0, w.split_list))
             return false;
-    } else {
-        for (uint32_t q = grid_stride_start(); q < n; q += grid_stride()) w.split_rank[q] = 0u;
-        if (blockIdx.x == 0 && threadIdx.x == 0) cin->n_split = 0u;
+        if (blockIdx.x == 0 && threadIdx.x == 0) split_guard_body(c, cin, cin->n_split, a.cap);
+        if (!grid_barrier(a, ++k, cin, cout)) return false;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) split_guard_body(c, cin, a.cap);
-    if (!grid_barrier(a, ++k, cin, cout)) return false;
     // no merge stage when the energy pass found no candidate (read after its barrier)
     if (c.use_merge && (c.merge_rule == SPH_MERGE_WAVELET_CELL || cin->merge_candidates)) {
         if (c.merge_rule == SPH_MERGE_SIBLING) merge_sibling_body<DIM>(c, cin, in, w);
@@ -249,12 +241,9 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
     if (cin->removed_flags) {
         if (!grid_scan<uint32_t>(a, k, cin, cout, w.removed_c, w.removed_rank, n, &cin->n_removed, 0, nullptr))
             return false;
-    } else {
-        for (uint32_t q = grid_stride_start(); q < n; q += grid_stride()) w.removed_rank[q] = 0u;
-        if (blockIdx.x == 0 && threadIdx.x == 0) cin->n_removed = 0u;
+        if (!grid_barrier(a, ++k, cin, cout)) return false;
     }
-    if (!grid_barrier(a, ++k, cin, cout)) return false;
-    write_body<DIM>(c, cin, cout, in, out, w, true, true);
+    write_body<DIM>(c, cin, cout, in, out, w, true);
     return true;
 }
 

@@ -148,8 +148,9 @@ __global__ void __launch_bounds__(kThreads) k_tape_record(const Counters *__rest
         t.spos[s] = w.spos[s]; t.svel[s] = w.svel[s]; t.sev[s] = w.sev[s];
         t.saux[s] = w.saux[s]; t.sacc[s] = w.sacc_n[s];
         t.spos_n[s] = w.spos_n[s]; t.svel_n[s] = w.svel_n[s]; t.sev_n[s] = w.sev_n[s];
-        t.split_c[s] = w.split_c[s]; t.split_rank[s] = w.split_rank[s];
-        t.removed_c[s] = w.removed_c[s]; t.removed_rank[s] = w.removed_rank[s];
+        // a step without splits or removals wrote no ranks
+        t.split_c[s] = w.split_c[s]; t.split_rank[s] = cnt->split_flags ? w.split_rank[s] : 0u;
+        t.removed_c[s] = w.removed_c[s]; t.removed_rank[s] = cnt->removed_flags ? w.removed_rank[s] : 0u;
         t.mpos[s] = w.mpos[s]; t.mvel[s] = w.mvel[s]; t.mev[s] = w.mev[s];
         if (w.nscenes) t.sscene[s] = w.sscene[s];
     }

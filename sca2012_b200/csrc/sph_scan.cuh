@@ -3,8 +3,9 @@
 // never needs the host to learn the count (the reference syncs on two
 // thrust::reduce calls per step, SPH-3D-2/sph_system.cu:1639,1836).
 //
-// Two launches: per-block chunk totals, then per-block rescans, each block
-// summing the block totals before its own (scan_phase23).  The grid is fixed
+// One launch of one thread-block cluster for small inputs (cluster_scan_body,
+// below).  Otherwise two launches: per-block chunk totals, then per-block
+// rescans, each block summing the block totals before its own (scan_phase23).  The grid is fixed
 // at launch (kScanBlocks); each block takes a contiguous chunk of
 // ceil(len/kScanBlocks) elements, so the traffic is two reads and one write
 // of the input.  (The three-launch form, with one block scanning the totals
@@ -89,7 +90,8 @@ __device__ __forceinline__ void scan_phase1_body(const T *in, uint32_t len, T *b
 }
 
 // skip_if_zero (optional): a count of the nonzero inputs; at 0 the scan is
-// all zeros, which scan_phase23 writes without reading the input.
+// all zeros, and scan_phase23 writes the total only (the readers of the ranks
+// test the same count).
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) scan_phase1(const T *__restrict__ in, const uint32_t *len_ptr,
                                                            uint32_t len_const, T *__restrict__ block_tot,
@@ -250,9 +252,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_phase23(const T *__restrict
                                                             const uint32_t *skip_if_zero = nullptr)
 {
     const uint32_t len = len_ptr ? *len_ptr : len_const;
-    if (skip_if_zero && *skip_if_zero == 0u) {   // every input is zero: so is every output
-        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x)
-            out[i] = zero_of<T>();
+    if (skip_if_zero && *skip_if_zero == 0u) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             if (grand) *grand = zero_of<T>();
             if (out_total_at_len) out[len] = zero_of<T>();
@@ -260,6 +260,120 @@ __global__ void __launch_bounds__(kScanThreads) scan_phase23(const T *__restrict
         return;
     }
     scan_phase23_body<T>(in, out, len, block_tot, grand, out_total_at_len, list);
+}
+
+// ------------------------------------------------------------ one-launch scan
+// The whole scan by ONE thread-block cluster: each warp sums its contiguous
+// segment, the blocks exchange their totals through distributed shared memory
+// and meet once at the hardware cluster barrier (nothing polls), and each warp
+// rescans its segment, 128 elements (four per lane) at a time.  Two reads and
+// one write of the input, like the two launches above, by 16 SMs: the launch
+// and the drain between the two are saved, which is what a scan of some 100,000
+// elements mostly costs (the host takes it up to the size where 16 SMs run out
+// of bandwidth; figures there).
+constexpr int kClusterScanThreads = 1024;
+constexpr int kClusterScanBlocks = 16;   // 8 where 16 cannot be scheduled
+
+struct ClusterScan {
+    uint32_t *in;                   // cleared behind the scan when `clear` is set
+    uint32_t *out;
+    const uint32_t *len_ptr;        // device length, or null:
+    uint32_t len;
+    uint32_t *grand;                // total, or null
+    uint32_t *list;                 // list[out[i]] = i for in[i] != 0, or null
+    const uint32_t *skip_if_zero;   // a device count of the nonzero inputs, or null; at 0 only the
+                                    // total is written (the readers of `out` test the count too)
+    int total_at_len;               // out[len] = total
+    int clear;
+};
+
+// Called by every thread of the cluster; returns the total to all of them.
+__device__ __forceinline__ uint32_t cluster_scan_body(const ClusterScan &j)
+{
+    __shared__ uint32_t warp_off[kClusterScanThreads / 32 + 1];
+    __shared__ uint32_t block_tot[kClusterScanBlocks];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr uint32_t nw = kClusterScanThreads / 32;
+    const uint32_t nb = gridDim.x, rank = blockIdx.x;   // the grid is one cluster
+    const uint32_t len = j.len_ptr ? *j.len_ptr : j.len;
+    const uint32_t seg = ((len + nb * nw - 1) / (nb * nw) + 127u) & ~127u;
+    const uint64_t b64 = (uint64_t)(rank * nw + warp) * seg;
+    const uint32_t b = (uint32_t)min((uint64_t)len, b64), e = (uint32_t)min((uint64_t)len, b64 + seg);
+    auto load4 = [&](uint32_t i) -> uint4 {   // in[i .. i + 3], zeros from e on
+        if (i + 4u <= e) return *reinterpret_cast<const uint4 *>(j.in + i);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (i < e) v.x = j.in[i];
+        if (i + 1u < e) v.y = j.in[i + 1u];
+        if (i + 2u < e) v.z = j.in[i + 2u];
+        return v;
+    };
+    uint32_t acc = 0;
+#pragma unroll 4
+    for (uint32_t i = b + 4u * lane; i < e; i += 128u) {
+        const uint4 v = load4(i);
+        acc += v.x + v.y + v.z + v.w;
+    }
+    acc = __reduce_add_sync(0xffffffffu, acc);
+    if (lane == 0) warp_off[warp + 1] = acc;
+    __syncthreads();
+    if (warp == 0) {   // exclusive offsets of the warps, block total last
+        uint32_t v = warp_off[lane + 1];
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, v, d);
+            if (lane >= d) v += o;
+        }
+        warp_off[lane + 1] = v;
+        if (lane == 0) warp_off[0] = 0u;
+        const uint32_t total = __shfl_sync(0xffffffffu, v, 31);
+        if ((uint32_t)lane < nb) {   // this block's total into every block's table
+            uint32_t dst;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(dst) : "r"((uint32_t)__cvta_generic_to_shared(block_tot + rank)), "r"(lane));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(dst), "r"(total) : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    uint32_t off = 0, all = 0;
+    for (uint32_t r = 0; r < nb; ++r) {
+        const uint32_t v = block_tot[r];
+        all += v;
+        if (r < rank) off += v;
+    }
+    uint32_t carry = off + warp_off[warp];
+#pragma unroll 2
+    for (uint32_t base = b; base < e; base += 128u) {
+        const uint32_t i = base + 4u * lane;
+        const uint4 v = load4(i);
+        const uint32_t own = v.x + v.y + v.z + v.w;
+        uint32_t inc = own;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
+        }
+        const uint32_t x0 = carry + inc - own, x1 = x0 + v.x, x2 = x1 + v.y, x3 = x2 + v.z;
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+        if (i + 4u <= e) {
+            *reinterpret_cast<uint4 *>(j.out + i) = make_uint4(x0, x1, x2, x3);
+            if (j.clear) *reinterpret_cast<uint4 *>(j.in + i) = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+            const uint32_t x[3] = {x0, x1, x2};
+            for (uint32_t u = 0; u < 3u && i + u < e; ++u) {
+                j.out[i + u] = x[u];
+                if (j.clear) j.in[i + u] = 0u;
+            }
+        }
+        if (j.list) {
+            if (v.x) j.list[x0] = i;
+            if (v.y) j.list[x1] = i + 1u;
+            if (v.z) j.list[x2] = i + 2u;
+            if (v.w) j.list[x3] = i + 3u;
+        }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        if (j.grand) *j.grand = all;
+        if (j.total_at_len) j.out[len] = all;
+    }
+    return all;
 }
 
 template <typename T>
