@@ -821,8 +821,9 @@ __device__ __forceinline__ void force_integrate_body(const sph_config &c, Counte
                 lap = __fmaf_rn(ilap * mrj * x, __fsub_rn(r2, c.lapc_three_quarters * x), lap);
             if (SAME.value) {
                 if (ok) sums(iin ? tg : 0.0f, tp, tv);
-            } else {   // a zero term leaves a sum as it is
-                sums(ok && iin ? tg : 0.0f, ok ? tp : 0.0f, ok ? tv : 0.0f);
+            } else {
+                const float tgs = ok && iin ? tg : 0.0f;   // a zero term leaves a sum as it is
+                if (ok) sums(tgs, tp, tv);
             }
         };
         auto pair = [&](uint32_t t) { pair_ab(true, w.fnb_a[t], w.fnb_b[t], std::false_type()); };

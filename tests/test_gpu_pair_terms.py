@@ -73,3 +73,23 @@ def test_single_pair(gpu, gap):
         dens, press, _ = O.density(c, pos, level, idx, cs, ce)
         got = O.force(c, pos, vel, level, dens, press, idx, cs, ce)
         check_close("force", out["acc"], np.asarray(got[0])[:, :3])
+
+
+@pytest.mark.parametrize("levels", [(1,), (1, 2)])
+def test_rejected_neighbour_with_nan_velocity_adds_nothing(gpu, levels):
+    """A listed neighbour outside the pair test contributes nothing, whatever
+    its velocity holds: the list path keeps the walk's bits."""
+    cfg, pos, vel, level = _cloud(3, 400, levels, 3.5, seed=11)
+    vel[::40] = np.nan
+    outs = []
+    for walk in (0, 1):
+        c = cfg.copy()
+        c.walk_only = walk
+        s = sph.Solver(c)
+        s.set_state(dict(pos=pos, vel=np.zeros_like(vel), ev=vel, level=level))
+        s.step(1)
+        outs.append(s.get_state())
+        s.close()
+    assert np.isnan(outs[0]["acc"]).any() and np.isfinite(outs[0]["acc"]).all(-1).any()
+    for f in ("acc", "surface", "pos", "energy"):
+        assert np.array_equal(outs[0][f], outs[1][f], equal_nan=True), f
