@@ -173,13 +173,21 @@ uint32_t grid_st(const sph_handle *h, uint32_t work, int stage)
     return std::max(1u, std::min(b, cap));
 }
 
+// Threads the merge pass asks for: one per particle for the split groups, a
+// warp per kMergeCellsMin cells for the per-cell rules.
+uint32_t merge_work(const sph_handle *h)
+{
+    if (h->cfg.merge_rule == SPH_MERGE_SIBLING) return h->n_ub;
+    return (uint32_t)std::min<uint64_t>((uint64_t)h->ncells * 32u / kMergeCellsMin, 1u << 31);
+}
+
 // Launch key of the step: every stage's grid and block size (a captured
 // graph is valid while it is unchanged).
 uint64_t launch_key(const sph_handle *h)
 {
     uint64_t k = 1469598103934665603ull;
     for (int st = 0; st < SPH_TUNE_STAGES; ++st) {
-        const uint32_t work = st == SPH_TUNE_MERGE ? h->ncells : h->n_ub;
+        const uint32_t work = st == SPH_TUNE_MERGE ? merge_work(h) : h->n_ub;
         k = (k ^ grid_st(h, work, st)) * 1099511628211ull;
         k = (k ^ (h->tune_bs[st] * 2u + (h->tune_minb[st] ? 1u : 0u))) * 1099511628211ull;
     }
@@ -441,9 +449,9 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
         }
         stage(h, "scan_split");
     }
-    if (c.use_merge) {   // one lane per cell, a warp scans 32 cells at a time
+    if (c.use_merge) {
         SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_MERGE],
-                      k_merge<DIM, B><<<grid_st(h, h->ncells, SPH_TUNE_MERGE), B, 0, s>>>(c, cin, in, w, h->ncells,
+                      k_merge<DIM, B><<<grid_st(h, merge_work(h), SPH_TUNE_MERGE), B, 0, s>>>(c, cin, in, w, h->ncells,
                                                                                           h->cap));
         h->last_launches += 1;
         stage(h, "merge");

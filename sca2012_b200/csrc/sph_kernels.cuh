@@ -1224,6 +1224,12 @@ __global__ void __launch_bounds__(kClusterScanThreads) k_split_ranks(ClusterScan
 // into the first, with V = m/rho weights (level already set to 1 for the
 // survivor, :1742-1777) or the plain mean in 2D.
 constexpr int kMergeListMax = 256;   // eligible members held per warp in shared memory
+// Cells per warp: as few as give every warp of the grid its share, from 2 to
+// 32.  32 cells of a dense fluid (14 particles per cell) hold more eligible
+// members than the list, and the warp then takes its cells one at a time; the
+// 47,564-particle four-way frame (16,000 cells) spent 136 us so, and 73, 34, 20
+// and 15 us with 16, 8, 4 and 2 cells.  A large empty grid keeps 32.
+constexpr uint32_t kMergeCellsMin = 2, kMergeCellsMax = 32;
 
 template <int DIM>
 __device__ __forceinline__ int merge_eligible(const sph_config &c, const WorkPtrs &w, uint32_t t,
@@ -1325,10 +1331,11 @@ __device__ __forceinline__ void merge_body(const sph_config &c, Counters *cnt, c
         }
         return split_score(c, eq, sq);
     };
-    // each warp takes 32 consecutive cells at a time; their members are one
+    // each warp takes `per` consecutive cells at a time; their members are one
     // contiguous slot range, tested 32 slots at a time
-    for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + wib) * 32u; base < ncells; base += warps_total * 32u) {
-        const uint32_t cend = min(base + 32u, ncells);
+    const uint32_t per = min(max((ncells + warps_total - 1u) / warps_total, kMergeCellsMin), kMergeCellsMax);
+    for (uint32_t base = (blockIdx.x * (blockDim.x >> 5) + wib) * per; base < ncells; base += warps_total * per) {
+        const uint32_t cend = min(base + per, ncells);
         const uint32_t sb = w.cell_off[base], se = w.cell_off[cend];
         // every eligible member is listed with its cell and its rank among
         // the cell's eligible members (cells are contiguous in slot order; the
