@@ -43,10 +43,6 @@ struct TapeStep {
     uint32_t *sscene;                         // scene per slot (batched scenes)
 };
 
-struct StepCounts {
-    uint32_t n, n_split, n_removed, split_on;
-};
-
 struct AdjPtrs {
     const float4 *gx_out, *gv_out, *gev_out;  // canonical, the next step's count
     float4 *gx_in, *gv_in, *gev_in;           // canonical, this step's count
@@ -96,12 +92,13 @@ __global__ void __launch_bounds__(kThreads) adj_write(sph_config c, StepCounts k
     for (uint32_t i = grid_stride_start(); i < k.n; i += grid_stride()) {
         const uint32_t s = t.inv[i];
         const uint32_t sp = k.split_on & t.split_c[i];
-        const uint32_t rm = t.removed_c[i];
-        const uint32_t L = t.merge_to[s];
+        // a step without removals wrote no removal ranks
+        const uint32_t rm = k.n_removed ? t.removed_c[i] : 0u;
+        const uint32_t L = k.n_removed ? t.merge_to[s] : kEmpty;
         float4 gx = make_float4(0.f, 0.f, 0.f, 0.f), gv = gx, ge = gx;
         float gr = 0.0f;
         if (!rm && L == kEmpty) {   // own record: the value itself (+ a constant shift when split)
-            const uint32_t o = i - t.removed_rank[i];
+            const uint32_t o = i - (k.n_removed ? t.removed_rank[i] : 0u);
             axpy3(gx, 1.0f, a.gx_out[o]); axpy3(gv, 1.0f, a.gv_out[o]); axpy3(ge, 1.0f, a.gev_out[o]);
         }
         if (sp) {                   // children copy the pre-split values
@@ -135,11 +132,16 @@ __global__ void __launch_bounds__(kThreads) adj_write(sph_config c, StepCounts k
 
 // ---------------------------------------------------------------- integrate + walls
 template <int DIM>
-__global__ void __launch_bounds__(kThreads) adj_integrate(sph_config c, StepCounts k, TapeStep t, AdjPtrs a)
+__global__ void __launch_bounds__(kThreads) adj_integrate(sph_config c, StepCounts k, TapeStep t, WorkPtrs w, AdjPtrs a)
 {
     const float dt = c.time_step, damp = c.wall_damping;
     for (uint32_t s = grid_stride_start(); s < k.n; s += grid_stride()) {
-        const float mi = c.mass[lv(t.spos[s].w)];
+        // a neighbour's values for the force pairs in two records, as the
+        // density pass leaves them for the forward force
+        const float4 ps = t.spos[s], as = t.saux[s], es = t.sev[s];
+        w.fnb_a[s] = make_float4(ps.x, ps.y, ps.z, as.z);
+        w.fnb_b[s] = make_float4(lv(ps.w) ? -as.w : as.w, es.x, es.y, es.z);
+        const float mi = c.mass[lv(ps.w)];
         const float im = 1.0f / mi;
         const uint32_t flags = t.wall[s];
         const float4 gx2 = a.gx2[s], ge2 = a.gev2[s];
@@ -164,58 +166,26 @@ __global__ void __launch_bounds__(kThreads) adj_integrate(sph_config c, StepCoun
 
 // ---------------------------------------------------------------- force pairs
 // ---------------------------------------------------------------- candidate lists
-// The neighbour candidate list of a taped step, rebuilt from the tape: the
-// step's start-of-step positions and cell ranges give the same stencil walk,
-// and so the same entries in the same order, as the forward density pass
-// recorded (every neighbour within (1 + margin) h_max).
+// The neighbour list of a taped step, rebuilt from the tape by the forward
+// density pass's walk over the step's positions and cell ranges: every
+// neighbour within h_max, in walk order.  (The forward lists' margin serves the
+// energy pass, which has no adjoint.)  Bound as the density pass; 38,500
+// particles: 33 us as a walk that tests and stores one candidate at a time, 20.
 template <int DIM>
-__global__ void __launch_bounds__(kThreads) adj_lists(sph_config c, StepCounts k, TapeStep t, WorkPtrs w)
+__global__ void __launch_bounds__(128) adj_lists(sph_config c, StepCounts k, TapeStep t, WorkPtrs w)
 {
-    const float re2 = energy_list_r2(c);
-    for (uint32_t s = grid_stride_start(); s < k.n; s += grid_stride()) {
-        const float4 pi = t.spos[s];
-        const uint32_t key = t.skey[s];
-        uint3 q;
-        q.x = key % c.ncell[0];
-        q.y = (key / c.ncell[0]) % c.ncell[1];
-        q.z = DIM == 3 ? key / (c.ncell[0] * c.ncell[1]) : 0u;
-        uint32_t nl = 0;
-        auto add = [&](uint32_t j, float4 pj) {   // j != s
-            float dx, dyy, dzz;
-            if (r2_of<DIM>(pj, pi, dx, dyy, dzz) < re2) {
-                if (nl < kNbrListCap) w.nlist[nl_at(w, s, nl)] = j;
-                ++nl;
-            }
-        };
-        auto range = [&](uint32_t b, uint32_t e) {
-            uint32_t j = b;
-            for (; j + 4 <= e; j += 4) {
-                const float4 p0 = t.spos[j], p1 = t.spos[j + 1], p2 = t.spos[j + 2], p3 = t.spos[j + 3];
-                add(j, p0);
-                add(j + 1, p1);
-                add(j + 2, p2);
-                add(j + 3, p3);
-            }
-            for (; j < e; ++j) add(j, t.spos[j]);
-        };
-#pragma unroll 1
-        for (int dz = (DIM == 3 ? -1 : 0); dz <= (DIM == 3 ? 1 : 0); ++dz)
-#pragma unroll 1
-            for (int dy = -1; dy <= 1; ++dy) {
-                uint32_t b, e;
-                if (!row_range<DIM>(c, t.cell_off, q, dy, dz, b, e)) continue;
-                if (dy == 0 && dz == 0) {
-                    range(b, s);
-                    range(s + 1u, e);
-                } else {
-                    range(b, e);
-                }
-            }
-        w.ncnt[s] = nl;
-    }
+    __shared__ DensSmem<kDensCap<128>> smem[4];
+    w.spos = t.spos;
+    w.skey = t.skey;
+    w.cell_off = t.cell_off;
+    density_walk<DIM, 128, true, false, kDensCap<128>, kDensFlush<128>, true>(c, nullptr, k.n, w, smem);
 }
 
-// The pairs come from the step's candidate list, filtered by the forward
+// Bound: the latency of the neighbour gathers.  A neighbour's values are the
+// forward pass's two records (adj_integrate leaves them) and its force adjoint,
+// three 16-byte loads issued before the terms instead of four behind the test;
+// 38,500 particles: 41 -> 26 us.
+// The pairs come from the step's neighbour list, filtered by the forward
 // pass's test, or, when a lane's list overflowed, from the warp-lockstep
 // stencil walk (warp_pairs).  Either way each lane adds its pairs in walk
 // order, so the sums do not depend on the path or on which particles share
@@ -238,14 +208,14 @@ __global__ void __launch_bounds__(kThreads) adj_force(sph_config c, StepCounts k
         const uint32_t sid = scene_of(w, t, s);
         const float visc = w.nscenes ? w.scene_tab[2 * sid].w : c.viscosity;
         const float gas = w.nscenes ? w.scene_tab[2 * sid + 1].w : c.gas_constant;
-        const uint32_t key = t.skey[s];
-        uint3 q;
-        q.x = key % c.ncell[0];
-        q.y = (key / c.ncell[0]) % c.ncell[1];
-        q.z = DIM == 3 ? key / (c.ncell[0] * c.ncell[1]) : 0u;
+        const uint3 q = cell_of_key<DIM>(c, t.skey[s]);
         const float cut0 = fmaxf(hi2, c.kernel2[0]), cut1 = fmaxf(hi2, c.kernel2[1]);
         float4 gx = make_float4(0.f, 0.f, 0.f, 0.f), ge = gx;
         float gA = 0.f, gV = 0.f, gmu = 0.f;
+        const float jspk0 = c.kernel_h6_twice ? c.spiky[0] / c.kernel6[0] : c.spiky[0];
+        const float jspk1 = c.kernel_h6_twice ? c.spiky[1] / c.kernel6[1] : c.spiky[1];
+        const float jvis0 = c.kernel_h6_twice ? c.visco[0] / c.kernel6[0] : c.visco[0];
+        const float jvis1 = c.kernel_h6_twice ? c.visco[1] / c.kernel6[1] : c.visco[1];
         // the forward pass's pairs: j != i, r^2 < max(h_i^2, h_j^2), r^2 >= close_r2
         auto accept = [&](uint32_t j, const float4 &pj) {
             float rx, ry, rz;
@@ -253,55 +223,71 @@ __global__ void __launch_bounds__(kThreads) adj_force(sph_config c, StepCounts k
             const float cut = pj.w == 1.0f ? cut0 : cut1;
             return j != s && r2 < cut && !(r2 < c.close_r2);
         };
-        auto pair = [&](uint32_t j) {
-            const float4 pj = t.spos[j];
+        // one pair (fa, fb: the neighbour's records, gfj: its force adjoint),
+        // added when `in` and the pair test holds; the terms without a branch,
+        // as in the forward force
+        auto pair = [&](bool in, const float4 fa, const float4 fb, const float4 gfj) {
             float rx, ry, rz;
-            const float r2 = r2_of<DIM>(pi, pj, rx, ry, rz);
-            const int lj = lv(pj.w);
-            const float r = __fsqrt_rn(r2);
-            const float ikr = __fsub_rn(hi, r), jkr = __fsub_rn(c.kernel[lj], r);
-            float S = 0.f, dS = 0.f, T = 0.f, dT = 0.f;
-            if (ikr > 0.0f) { S += ispk * ikr * ikr; dS -= 2.0f * ispk * ikr; T += ivis * ikr; dT -= ivis; }
-            if (jkr > 0.0f) {
-                const float jspk = c.kernel_h6_twice ? c.spiky[lj] / c.kernel6[lj] : c.spiky[lj];
-                const float jvis = c.kernel_h6_twice ? c.visco[lj] / c.kernel6[lj] : c.visco[lj];
-                S += jspk * jkr * jkr; dS -= 2.0f * jspk * jkr; T += jvis * jkr; dT -= jvis;
-            }
-            const float4 aj = t.saux[j], evj = t.sev[j], gfj = a.gf[j];
-            const float mm = mi * c.mass[lj];
-            const float Cp = mm * (ai.z + aj.z) * 0.5f;
-            const float ir = rsqrtf(r2);   // 1/r as the forward pass takes it
-            const float tp = Cp * S * ir, dtp = Cp * (dS - S * ir) * ir;
-            const float VV = ai.w * aj.w;
+            const float r2 = r2_of<DIM>(pi, fa, rx, ry, rz);
+            const bool lj = signbit(fb.x);
+            const bool ok = in && r2 < (lj ? cut1 : cut0) && !(r2 < c.close_r2);
+            const float ir = rsqrt_normal(r2), r = sqrt_of(r2, ir);   // as the forward pass takes them
+            const float ikr = __fsub_rn(hi, r), jkr = __fsub_rn(lj ? c.kernel[1] : c.kernel[0], r);
+            const float iq = ikr > 0.0f ? ikr : 0.0f, jq = jkr > 0.0f ? jkr : 0.0f;
+            const float jspk = lj ? jspk1 : jspk0, jvis = lj ? jvis1 : jvis0;
+            const float S = __fmaf_rn(ispk * iq, iq, jspk * jq * jq);
+            const float dS = -2.0f * __fmaf_rn(ispk, iq, jspk * jq);
+            const float T = __fmaf_rn(ivis, iq, jvis * jq);
+            const float dT = -((ikr > 0.0f ? ivis : 0.0f) + (jkr > 0.0f ? jvis : 0.0f));
+            const float mrj = fabsf(fb.x);
+            const float mm = mi * (lj ? c.mass[1] : c.mass[0]);
+            const float Cp = mm * __fadd_rn(ai.z, fa.w) * 0.5f;
+            const float tp = Cp * S * ir, dtp = Cp * __fmaf_rn(-S, ir, dS) * ir;
+            const float VV = ai.w * mrj;
             const float tv = VV * visc * 0.5f * T, dtv = VV * visc * 0.5f * dT;
-            const float4 D = sub3(gfi, gfj);
-            const float4 rv = make_float4(rx, ry, rz, 0.f);
-            const float4 dv = sub3(evj, evi);
-            const float Dr = dot3(D, rv), Ddv = dot3(D, dv);
-            const float coef = (Ddv * dtv - Dr * dtp) * ir;
-            axpy3(gx, -tp, D);
-            axpy3(gx, coef, rv);
-            axpy3(ge, -tv, D);
-            gA -= Dr * mm * 0.5f * S * ir;
-            gV += Ddv * aj.w * visc * 0.5f * T;
-            gmu += 0.25f * Ddv * VV * T;     // each unordered pair is visited from both ends
+            const float Dx = __fsub_rn(gfi.x, gfj.x), Dy = __fsub_rn(gfi.y, gfj.y), Dz = __fsub_rn(gfi.z, gfj.z);
+            const float vx = __fsub_rn(fb.y, evi.x), vy = __fsub_rn(fb.z, evi.y), vz = __fsub_rn(fb.w, evi.z);
+            const float Dr = __fmaf_rn(Dz, rz, __fmaf_rn(Dy, ry, __fmul_rn(Dx, rx)));
+            const float Ddv = __fmaf_rn(Dz, vz, __fmaf_rn(Dy, vy, __fmul_rn(Dx, vx)));
+            const float coef = __fmaf_rn(Ddv, dtv, -__fmul_rn(Dr, dtp)) * ir;
+            if (ok) {
+                gx.x = __fmaf_rn(coef, rx, __fmaf_rn(-tp, Dx, gx.x));
+                gx.y = __fmaf_rn(coef, ry, __fmaf_rn(-tp, Dy, gx.y));
+                gx.z = __fmaf_rn(coef, rz, __fmaf_rn(-tp, Dz, gx.z));
+                ge.x = __fmaf_rn(-tv, Dx, ge.x);
+                ge.y = __fmaf_rn(-tv, Dy, ge.y);
+                ge.z = __fmaf_rn(-tv, Dz, ge.z);
+                gA = __fmaf_rn(-Dr, mm * 0.5f * S * ir, gA);
+                gV = __fmaf_rn(Ddv, mrj * visc * 0.5f * T, gV);
+                gmu = __fmaf_rn(0.25f * Ddv, VV * T, gmu);   // each unordered pair is visited from both ends
+            }
         };
         const unsigned full = 0xffffffffu;
         const uint32_t nf = valid && w.nlist ? w.ncnt[s] : 0u;
         if (__all_sync(full, w.nlist != nullptr && nf <= kNbrListCap)) {
             const uint32_t m = __reduce_max_sync(full, nf);
-            if (4 < m) prefetch_l2(w.nlist + nl_at(w, s, 4));
+            const uint4 *lp = reinterpret_cast<const uint4 *>(w.nlist) + s;   // chunk j at lp[j * nl_stride]
+            uint4 nxt = nf ? *lp : make_uint4(s, s, s, s);
+            if (4 < m) prefetch_l2(lp + w.nl_stride);
             for (uint32_t kk = 0; kk < m; kk += 4) {
-                if (kk + 8 < m) prefetch_l2(w.nlist + nl_at(w, s, kk + 8));   // two rounds ahead
-                const uint4 t4 = *reinterpret_cast<const uint4 *>(w.nlist + nl_at(w, s, kk));
+                const uint4 t4 = nxt;
+                lp += w.nl_stride;
+                if (kk + 8 < m) prefetch_l2(lp + w.nl_stride);   // two rounds ahead
+                if (kk + 4 < nf) nxt = *lp;
                 const uint32_t tt[4] = {kk < nf ? t4.x : s, kk + 1 < nf ? t4.y : s, kk + 2 < nf ? t4.z : s,
                                         kk + 3 < nf ? t4.w : s};
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (kk + u < nf && accept(tt[u], t.spos[tt[u]])) pair(tt[u]);
+                for (int q = 0; q < 4; q += 2) {   // two neighbours' loads in flight
+                    const float4 a0 = w.fnb_a[tt[q]], a1 = w.fnb_a[tt[q + 1]];
+                    const float4 b0 = w.fnb_b[tt[q]], b1 = w.fnb_b[tt[q + 1]];
+                    const float4 g0 = a.gf[tt[q]], g1 = a.gf[tt[q + 1]];
+                    pair(kk + q < nf, a0, b0, g0);
+                    pair(kk + q + 1 < nf, a1, b1, g1);
+                }
             }
         } else {
-            warp_pairs<DIM>(c, t.cell_off, t.spos, valid, q, smem[wib], accept, pair);
+            auto walked = [&](uint32_t j) { pair(true, w.fnb_a[j], w.fnb_b[j], a.gf[j]); };
+            warp_pairs<DIM>(c, t.cell_off, t.spos, valid, q, smem[wib], accept, walked);
         }
         if (!valid) continue;
         // p = gas ((rho/rho0)^3 - 1); A = p / rho^2; V = m / rho
@@ -320,6 +306,8 @@ __global__ void __launch_bounds__(kThreads) adj_force(sph_config c, StepCounts k
 }
 
 // ---------------------------------------------------------------- density pairs
+// Both terms of a neighbour from two loads issued before either is needed, the
+// next list chunk a round ahead; 38,500 particles: 23 -> 13 us.
 template <int DIM>
 __global__ void __launch_bounds__(kThreads) adj_density(sph_config c, StepCounts k, TapeStep t, WorkPtrs w,
                                                         AdjPtrs a)
@@ -330,60 +318,65 @@ __global__ void __launch_bounds__(kThreads) adj_density(sph_config c, StepCounts
         const int li = lv(pi.w);
         const float h2 = c.kernel2[li], w6 = c.poly6[li], mi = c.mass[li];
         const float gri = a.grho[s];
-        const uint32_t key = t.skey[s];
-        uint3 q;
-        q.x = key % c.ncell[0];
-        q.y = (key / c.ncell[0]) % c.ncell[1];
-        q.z = DIM == 3 ? key / (c.ncell[0] * c.ncell[1]) : 0u;
+        // per neighbour level: the factors of its term in rho_i and of this
+        // particle's in rho_j
+        const float ci0 = gri * c.mass[0] * w6, ci1 = gri * c.mass[1] * w6;
+        const float cj0 = mi * c.poly6[0], cj1 = mi * c.poly6[1];
+        const float k0 = c.kernel2[0], k1 = c.kernel2[1];
         float4 gx = a.gxd[s];
-        auto visit = [&](uint32_t j, float4 pj) {   // j != s
+        // both terms of one neighbour j != s (gr: its rho adjoint), without a
+        // branch; added when `in` and the density pass takes the pair
+        auto visit = [&](bool in, const float4 pj, float gr) {
             float dx, dy_, dz_;
             const float r2 = r2_of<DIM>(pj, pi, dx, dy_, dz_);   // d = x_j - x_i
-            if (r2 < skip) return;
-            const int lj = lv(pj.w);
-            float acc = 0.0f;
-            if (r2 < h2) {          // term of rho_i
-                const float x = h2 - r2;
-                acc += gri * c.mass[lj] * w6 * x * x;
-            }
-            const float hj2 = c.kernel2[lj];
-            if (r2 < hj2) {         // term of rho_j
-                const float x = hj2 - r2;
-                acc += a.grho[j] * mi * c.poly6[lj] * x * x;
-            }
+            const bool l1 = pj.w == 1.0f;
+            const float hj2 = l1 ? k0 : k1;
+            const float xi = h2 - r2, xj = hj2 - r2;
+            const float ti = (l1 ? ci0 : ci1) * xi * xi, tj = gr * (l1 ? cj0 : cj1) * xj * xj;
             // d/dx_i (h^2 - r^2)^3 = -6 (h^2 - r^2)^2 (x_i - x_j) = +6 (...)^2 d
-            gx.x += 6.0f * acc * dx; gx.y += 6.0f * acc * dy_; gx.z += 6.0f * acc * dz_;
+            const float acc = 6.0f * __fadd_rn(r2 < h2 ? ti : 0.0f, r2 < hj2 ? tj : 0.0f);
+            if (in && !(r2 < skip)) {
+                gx.x = __fmaf_rn(acc, dx, gx.x);
+                gx.y = __fmaf_rn(acc, dy_, gx.y);
+                gx.z = __fmaf_rn(acc, dz_, gx.z);
+            }
         };
         // slot order, four candidates' loads in flight; the own row around s
         auto range = [&](uint32_t b, uint32_t e) {
             uint32_t j = b;
             for (; j + 4 <= e; j += 4) {
                 const float4 p0 = t.spos[j], p1 = t.spos[j + 1], p2 = t.spos[j + 2], p3 = t.spos[j + 3];
-                visit(j, p0);
-                visit(j + 1, p1);
-                visit(j + 2, p2);
-                visit(j + 3, p3);
+                const float g0 = a.grho[j], g1 = a.grho[j + 1], g2 = a.grho[j + 2], g3 = a.grho[j + 3];
+                visit(true, p0, g0);
+                visit(true, p1, g1);
+                visit(true, p2, g2);
+                visit(true, p3, g3);
             }
-            for (; j < e; ++j) visit(j, t.spos[j]);
+            for (; j < e; ++j) visit(true, t.spos[j], a.grho[j]);
         };
-        // the step's candidate list holds every pair with a term (r^2 below
+        // the step's neighbour list holds every pair with a term (r^2 below
         // h_i^2 or h_j^2), in walk order; an overflowed list walks
         const uint32_t nl = w.nlist ? w.ncnt[s] : kEmpty;
         if (nl <= kNbrListCap) {
-            uint32_t kk = 0;
-            for (; kk + 4 <= nl; kk += 4) {
-                const uint4 t4 = *reinterpret_cast<const uint4 *>(w.nlist + nl_at(w, s, kk));
-                const float4 p0 = t.spos[t4.x], p1 = t.spos[t4.y], p2 = t.spos[t4.z], p3 = t.spos[t4.w];
-                visit(t4.x, p0);
-                visit(t4.y, p1);
-                visit(t4.z, p2);
-                visit(t4.w, p3);
-            }
-            for (; kk < nl; ++kk) {
-                const uint32_t j = w.nlist[nl_at(w, s, kk)];
-                visit(j, t.spos[j]);
+            const uint4 *lp = reinterpret_cast<const uint4 *>(w.nlist) + s;   // chunk j at lp[j * nl_stride]
+            uint4 nxt = nl ? *lp : make_uint4(s, s, s, s);
+            for (uint32_t kk = 0; kk < nl; kk += 4) {
+                const uint4 t4 = nxt;
+                lp += w.nl_stride;
+                if (kk + 4 < nl) nxt = *lp;
+                const uint32_t tt[4] = {t4.x, kk + 1 < nl ? t4.y : s, kk + 2 < nl ? t4.z : s, kk + 3 < nl ? t4.w : s};
+                float4 pj[4];
+                float gr[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    pj[u] = t.spos[tt[u]];
+                    gr[u] = a.grho[tt[u]];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) visit(kk + u < nl, pj[u], gr[u]);
             }
         } else {
+            const uint3 q = cell_of_key<DIM>(c, t.skey[s]);
 #pragma unroll 1
             for (int dz = (DIM == 3 ? -1 : 0); dz <= (DIM == 3 ? 1 : 0); ++dz)
 #pragma unroll 1

@@ -53,6 +53,11 @@ struct Counters {
                            // pass (at 0 the merge pass has nothing to do and returns at once)
 };
 
+// Counts of one taped step, for its adjoint.
+struct StepCounts {
+    uint32_t n, n_split, n_removed, split_on;
+};
+
 struct CanonPtrs {
     float4 *pos, *vel, *ev, *acc;
     float *dens, *press, *energy, *surface;
@@ -83,6 +88,7 @@ struct WorkPtrs {
     uint32_t *merge_to;                  // taped steps only: slot -> its merge leader's slot
     float *mvs;                          // taped steps only: leader slot -> summed member volume
     uint32_t *wall;                      // taped steps only: wall contacts per slot
+    StepCounts *step_counts;             // taped steps only: where the write-out leaves the step's counts
     float4 *spos_lo, *spos_lo_n;         // low position parts per slot (compensated positions)
     uint32_t pos_comp;                   // the config's compensated_positions
     uint32_t *nlist, *ncnt;              // neighbour candidates (layout: nl_at), by the density pass
@@ -483,14 +489,15 @@ template <uint32_t CAP> struct DensSmem {
 // SKIP = false: the config skips no close pairs (density_skip_r2 == 0), so
 // the test !(r^2 < skip) is true for every r^2 and is left out.
 // FLUSH: the buffer entries a warp keeps free for its next chunk.
-template <int DIM, int BS, bool NC, bool SKIP, uint32_t CAP, uint32_t FLUSH>
-__device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt, const WorkPtrs &w,
+// LISTS: only the candidate lists, of every neighbour within h_max (no margin),
+// over n particles; cnt is not used.
+template <int DIM, int BS, bool NC, bool SKIP, uint32_t CAP, uint32_t FLUSH, bool LISTS = false>
+__device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt, uint32_t n, const WorkPtrs &w,
                                              DensSmem<CAP> *smem)
 {
     const unsigned full = 0xffffffffu;
-    const uint32_t n = cnt->n;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (!LISTS && blockIdx.x == 0 && threadIdx.x == 0) {
         cnt->disp2_max = 0u;   // the force pass takes the max
         cnt->n_split = cnt->n_removed = cnt->split_off = 0u;   // set by the rank scans a step runs
     }
@@ -517,7 +524,7 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
         const float m0 = c.mass[0], m1 = c.mass[1], skip = c.density_skip_r2;
         // (m_j * poly6) once per level: the same product the sum takes first
         const float mp0 = m0 * poly6, mp1 = m1 * poly6;
-        const float reach2 = rec ? energy_list_r2(c) : h2;
+        const float reach2 = LISTS ? fmaxf(c.kernel2[0], c.kernel2[1]) : rec ? energy_list_r2(c) : h2;
         const uint32_t self = s | (li ? kDensLevel2 : 0u);
         uint32_t *const lbase = rec ? w.nlist + (size_t)s * 4u : nullptr;
         float rho = 0.0f;
@@ -525,6 +532,7 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
         uint32_t at = col0;           // where the next buffer entry goes
         // one buffered pair into the sum: skip <= r^2 < h_i^2 (:394-417)
         auto take = [&](const uint2 ent) {
+            if (LISTS) return;
             const float r2 = __uint_as_float(ent.x);
             const float x = h2 - r2;
             const float x3 = x * x * x;
@@ -687,6 +695,10 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
         }
         drain(true);
         if (!valid) continue;
+        if (LISTS) {
+            w.ncnt[s] = nl;
+            continue;
+        }
         rho = __fadd_rn(rho, c.mass[li] * poly6 * c.kernel6[li]);   // self term
         float r = rho / c.rest_density;
         const float gas = w.nscenes ? w.scene_tab[2 * min(w.sscene[s], w.nscenes - 1u) + 1].w : c.gas_constant;
@@ -705,8 +717,8 @@ template <int DIM, int BS, bool NC, uint32_t CAP, uint32_t FLUSH>
 __device__ __forceinline__ void density_body(const sph_config &c, Counters *cnt, const WorkPtrs &w,
                                              DensSmem<CAP> *smem)
 {
-    if (c.density_skip_r2 == 0.0f) density_walk<DIM, BS, NC, false, CAP, FLUSH>(c, cnt, w, smem);
-    else density_walk<DIM, BS, NC, true, CAP, FLUSH>(c, cnt, w, smem);
+    if (c.density_skip_r2 == 0.0f) density_walk<DIM, BS, NC, false, CAP, FLUSH>(c, cnt, cnt->n, w, smem);
+    else density_walk<DIM, BS, NC, true, CAP, FLUSH>(c, cnt, cnt->n, w, smem);
 }
 
 // The standalone kernel is instantiated per SKIP (the host picks it): one
@@ -723,7 +735,7 @@ __global__ void __launch_bounds__(BS) k_density(sph_config c, Counters *__restri
 {
     extern __shared__ __align__(16) unsigned char dens_smem[];
     density_walk<DIM, BS, true, SKIP, kDensCap<BS>, kDensFlush<BS>>(
-        c, cnt, w, reinterpret_cast<DensSmem<kDensCap<BS>> *>(dens_smem));
+        c, cnt, cnt->n, w, reinterpret_cast<DensSmem<kDensCap<BS>> *>(dens_smem));
 }
 
 // ------------------------------------------------------------ 6. force + integrate
@@ -1496,6 +1508,7 @@ __device__ __forceinline__ void write_body(const sph_config &c, const Counters *
         cnt_next->split_flags = 0;
         cnt_next->removed_flags = 0;
         cnt_next->merge_candidates = 0;
+        if (w.step_counts) *w.step_counts = StepCounts{n, cnt->n_split, n_removed, cnt->split_off ? 0u : 1u};
     }
     // one thread per particle index: reads gather from the sorted slot, the
     // writes (survivors keep their order) stay coalesced
