@@ -87,6 +87,7 @@ __device__ __forceinline__ uint32_t scene_of(const WorkPtrs &w, const TapeStep &
 template <int DIM>
 __global__ void __launch_bounds__(kThreads) adj_write(sph_config c, StepCounts k, TapeStep t, AdjPtrs a)
 {
+    dependent_entry();
     const uint32_t ways = c.split_ways == 4 ? 4u : 2u, extra = ways - 1u;
     const float hs2 = c.kernel[1] / 2.0f;
     for (uint32_t i = grid_stride_start(); i < k.n; i += grid_stride()) {
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(kThreads) adj_write(sph_config c, StepCounts k
 template <int DIM>
 __global__ void __launch_bounds__(kThreads) adj_integrate(sph_config c, StepCounts k, TapeStep t, WorkPtrs w, AdjPtrs a)
 {
+    dependent_entry();
     const float dt = c.time_step, damp = c.wall_damping;
     for (uint32_t s = grid_stride_start(); s < k.n; s += grid_stride()) {
         // a neighbour's values for the force pairs in two records, as the
@@ -175,10 +177,11 @@ template <int DIM>
 __global__ void __launch_bounds__(128) adj_lists(sph_config c, StepCounts k, TapeStep t, WorkPtrs w)
 {
     __shared__ DensSmem<kDensCap<128>> smem[4];
+    dependent_entry();
     w.spos = t.spos;
     w.skey = t.skey;
     w.cell_off = t.cell_off;
-    density_walk<DIM, 128, true, false, kDensCap<128>, kDensFlush<128>, true>(c, nullptr, k.n, w, smem);
+    density_walk<DIM, 128, false, kDensCap<128>, kDensFlush<128>, true>(c, nullptr, k.n, w, smem);
 }
 
 // Bound: the latency of the neighbour gathers.  A neighbour's values are the
@@ -193,6 +196,7 @@ __global__ void __launch_bounds__(128) adj_lists(sph_config c, StepCounts k, Tap
 template <int DIM>
 __global__ void __launch_bounds__(kThreads) adj_force(sph_config c, StepCounts k, TapeStep t, WorkPtrs w, AdjPtrs a)
 {
+    dependent_entry();
     __shared__ WarpPairSmem smem[kThreads / 32];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t n = k.n;
@@ -312,6 +316,7 @@ template <int DIM>
 __global__ void __launch_bounds__(kThreads) adj_density(sph_config c, StepCounts k, TapeStep t, WorkPtrs w,
                                                         AdjPtrs a)
 {
+    dependent_entry();
     const float skip = c.density_skip_r2;
     for (uint32_t s = grid_stride_start(); s < k.n; s += grid_stride()) {
         const float4 pi = t.spos[s];

@@ -62,9 +62,10 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // for two nodes.  Each node still sums exactly its own stencil's particles in
 // its own walk order (a node whose cell differs from its partner's takes the
 // candidates of the joint row range that fall in its own range).
-__global__ void __launch_bounds__(kThreads) k_splat(sph_config c, const uint32_t *__restrict__ off,
-                                                   const float4 *__restrict__ pos, float *__restrict__ dens)
+__global__ void __launch_bounds__(kThreads) k_splat(sph_config c, const uint32_t *off,
+                                                   const float4 *pos, float *dens)
 {
+    dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
     const uint32_t GX = R / 2 + 1;   // groups {0}, {1, 2}, {3, 4}, ...
     const uint32_t G = GX * Cn * L;
@@ -134,9 +135,10 @@ __global__ void __launch_bounds__(kThreads) k_splat(sph_config c, const uint32_t
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const float *__restrict__ dens,
-                                                          float4 *__restrict__ normal)
+__global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const float *dens,
+                                                          float4 *normal)
 {
+    dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
     const uint32_t G = R * Cn * L;
     for (uint32_t g = grid_stride_start(); g < G; g += grid_stride()) {
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const f
     }
 }
 
-__device__ __forceinline__ uint32_t mc_cube_case(const sph_config &c, const float *__restrict__ dens, uint32_t x,
+__device__ __forceinline__ uint32_t mc_cube_case(const sph_config &c, const float *dens, uint32_t x,
                                                  uint32_t y, uint32_t z, uint32_t *corner_node)
 {
     const uint32_t R = c.ndens[0], Cn = c.ndens[1];
@@ -176,9 +178,10 @@ __device__ __forceinline__ uint32_t mc_tri_count(uint32_t flags)
     return k;
 }
 
-__global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float *__restrict__ dens,
-                                                      uint32_t *__restrict__ cnt)
+__global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float *dens,
+                                                      uint32_t *cnt)
 {
+    dependent_entry();
     const uint32_t Cm = c.ndens[1] - 1, Lm = c.ndens[2] - 1;
     const uint32_t Q = (c.ndens[0] - 1) * Cm * Lm;
     for (uint32_t q = grid_stride_start(); q < Q; q += grid_stride()) {
@@ -193,12 +196,13 @@ __global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float
 // places them (SPH-3D-2/sph_system.cpp:479-480), or linear interpolation at
 // the iso value when mc_interpolate is set; vertex normals are the mean of
 // the two node normals.
-__global__ void __launch_bounds__(kThreads) k_mc_emit(sph_config c, const float *__restrict__ dens,
-                                                     const float4 *__restrict__ normal,
-                                                     const uint32_t *__restrict__ cnt,
-                                                     const uint32_t *__restrict__ off, uint32_t max_tri,
-                                                     float *__restrict__ tri)
+__global__ void __launch_bounds__(kThreads) k_mc_emit(sph_config c, const float *dens,
+                                                     const float4 *normal,
+                                                     const uint32_t *cnt,
+                                                     const uint32_t *off, uint32_t max_tri,
+                                                     float *tri)
 {
+    dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1];
     const uint32_t Cm = Cn - 1, Lm = c.ndens[2] - 1;
     const uint32_t Q = (R - 1) * Cm * Lm;

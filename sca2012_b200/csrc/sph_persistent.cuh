@@ -42,8 +42,8 @@
 // A launch of several steps alternates the two state buffers and counters
 // as that many separate steps would (the grid is sized for the first step's
 // count, so only steps that cannot split share a launch).
-// No stage reads data through the non-coherent path (loads are NC = false),
-// since a stage reads what an earlier stage of the same launch wrote.
+// No stage reads data through the non-coherent path, since a stage reads what
+// an earlier stage of the same launch wrote.
 #pragma once
 #include <cstdint>
 #include "../../include/sph/sph.h"
@@ -208,17 +208,17 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
         return false;
     }
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    scatter_body<false>(cin, w);
+    scatter_body(cin, w);
     // no stage reads the counts after the scan: clear them for the next hash
     for (uint32_t q = grid_stride_start(); q < a.ncells; q += grid_stride()) w.cell_count[q] = 0u;
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    reorder_body<false>(cin, in, w);
+    reorder_body(cin, in, w);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    density_body<DIM, BS, false, kDensCapPersist, 8>(c, cin, w, dens);
+    density_body<DIM, BS, kDensCapPersist, 8>(c, cin, w, dens);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    force_integrate_body<DIM, BS, false>(c, cin, w, pair);
+    force_integrate_body<DIM, BS>(c, cin, w, pair);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    energy_split_body<DIM, BS, false>(c, cin, in, w, a.want_tv, pair);
+    energy_split_body<DIM, BS>(c, cin, in, w, a.want_tv, pair);
     if (!a.ranks) {
         write_hash_by_slot_body<DIM, BS>(c, cin, cout, in, out, w);
         return true;

@@ -215,10 +215,10 @@ template <int DIM> void sort_only(sph_handle *h)
     cudaMemsetAsync(w.cell_count, 0, sizeof(uint32_t) * h->ncells, s);
     h->counts_zero = false;
     h->counts_hashed = false;
-    k_hash<DIM><<<G, kThreads, 0, s>>>(c, cin, in, w);
+    launch(h, k_hash<DIM>, G, kThreads, 0, 0, c, cin, in, w);
     scan_u32(h, w.cell_count, w.cell_off, nullptr, h->ncells, h->scan_grand, 1, nullptr);
-    k_scatter<<<G, kThreads, 0, s>>>(cin, w);
-    k_reorder<<<G, kThreads, 0, s>>>(cin, in, w);
+    launch(h, k_scatter<>, G, kThreads, 0, 0, cin, w);
+    launch(h, k_reorder<>, G, kThreads, 0, 0, cin, in, w);
 }
 
 bool rollout_current(const sph_handle *h, const Rollout *r)
@@ -259,13 +259,13 @@ template <int DIM> int backward_impl(sph_handle *h, Rollout *r, float *d_vel0, f
             a.grho = r->grho;
             a.param = r->param;
             const uint32_t G = grid_for(h, k.n);
-            adj_write<DIM><<<G, kThreads, 0, s>>>(c, k, r->tape[l], a);
-            adj_integrate<DIM><<<G, kThreads, 0, s>>>(c, k, r->tape[l], w, a);
+            launch(h, adj_write<DIM>, G, kThreads, 0, 0, c, k, r->tape[l], a);
+            launch(h, adj_integrate<DIM>, G, kThreads, 0, 0, c, k, r->tape[l], w, a);
             // the step's candidate lists, rebuilt from its tape (the working
             // lists are free during the backward pass)
-            if (w.nlist) adj_lists<DIM><<<std::max(1u, (k.n + 127u) / 128u), 128, 0, s>>>(c, k, r->tape[l], w);
-            adj_force<DIM><<<G, kThreads, 0, s>>>(c, k, r->tape[l], w, a);
-            adj_density<DIM><<<G, kThreads, 0, s>>>(c, k, r->tape[l], w, a);
+            if (w.nlist) launch_pairs(h, adj_lists<DIM>, std::max(1u, (k.n + 127u) / 128u), 128, 0, c, k, r->tape[l], w);
+            launch_pairs(h, adj_force<DIM>, G, kThreads, 0, c, k, r->tape[l], w, a);
+            launch_pairs(h, adj_density<DIM>, G, kThreads, 0, c, k, r->tape[l], w, a);
             p ^= 1;
         }
     }
