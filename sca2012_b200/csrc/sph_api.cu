@@ -655,21 +655,6 @@ template <int DIM> int run_step_persistent(sph_handle *h, int nsteps)
     return cuda_check(h, "sph_step persistent");
 }
 
-void pack4(const float *src, int dim, uint32_t n, std::vector<float4> &dst, const uint32_t *level)
-{
-    dst.resize(n);
-    for (uint32_t i = 0; i < n; ++i) {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (src) {
-            v.x = src[(size_t)i * dim];
-            v.y = src[(size_t)i * dim + 1];
-            if (dim == 3) v.z = src[(size_t)i * dim + 2];
-        }
-        if (level) v.w = (float)level[i];
-        dst[i] = v;
-    }
-}
-
 void unpack4(const std::vector<float4> &src, int dim, uint32_t n, float *dst)
 {
     if (!dst) return;
@@ -688,23 +673,51 @@ uint32_t read_n(sph_handle *h)
     return n;
 }
 
+// Ends the replacement of the state by one of n particles: sets the device
+// count and waits for the handle's stream, so that the caller's arrays are free.
 void write_n(sph_handle *h, uint32_t n)
 {
-    Counters c0;
-    std::memset(&c0, 0, sizeof(c0));
-    cudaMemcpyAsync(&c0, &h->cnt[h->cur], sizeof(Counters), cudaMemcpyDeviceToHost, h->stream);
-    cudaStreamSynchronize(h->stream);
-    c0.n = n;
-    c0.error &= ~(1u << SPH_ERR_TIMEOUT);   // a new state: steps may run again after a timeout
-    cudaMemcpyAsync(&h->cnt[h->cur], &c0, sizeof(Counters), cudaMemcpyHostToDevice, h->stream);
-    // a new state: the persistent step's barrier states start clean (a
-    // timeout leaves its abort flag set) and the cell counts are cleared
-    // before its next launch
-    cudaMemsetAsync(h->gsync, 0, sizeof(GridSync) * 2, h->stream);
-    h->counts_zero = false;
+    static_assert(sizeof(GridSync) * 2 <= 32 * sizeof(uint32_t), "one warp clears both barrier states");
+    launch(h, k_set_count, 1, 32, 0, 0, h->cnt + h->cur, n, (uint32_t *)h->gsync,
+           (uint32_t)(sizeof(GridSync) * 2 / sizeof(uint32_t)));
+    h->counts_zero = false;      // the cell counts are cleared before the next launch
     h->counts_hashed = false;
-    h->outputs_pending = false;   // the caller wrote every field
+    h->outputs_pending = false;  // the caller wrote every field
     cudaStreamSynchronize(h->stream);
+}
+
+// Uploads the caller's vectors and levels as they are and unpacks them on the
+// device into the current state from particle `first` on.  The step's sorted
+// arrays, free between steps, hold the raw arrays meanwhile.
+void upload_vectors(sph_handle *h, uint32_t first, uint32_t n, const float *pos, const float *vel, const float *ev,
+                    const float *acc, const uint32_t *level)
+{
+    if (!n) return;
+    const int dim = (int)h->cfg.dim;
+    cudaStream_t s = h->stream;
+    auto raw = [&](const float *src, float4 *scratch) -> const float * {
+        if (!src) return nullptr;
+        cudaMemcpyAsync(scratch, src, sizeof(float) * (size_t)n * dim, cudaMemcpyHostToDevice, s);
+        return (const float *)scratch;
+    };
+    RawState r;
+    r.pos = raw(pos, h->w.spos);
+    r.vel = raw(vel, h->w.svel);
+    r.ev = raw(ev, h->w.sev);
+    r.acc = raw(acc, h->w.saux);
+    cudaMemcpyAsync(h->w.tmp, level, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s);
+    r.level = h->w.tmp;
+    const uint32_t G = grid_for(h, n);
+    if (dim == 3) launch(h, k_unpack_state<3>, G, kThreads, 0, 0, n, first, r, h->buf[h->cur]);
+    else launch(h, k_unpack_state<2>, G, kThreads, 0, 0, n, first, r, h->buf[h->cur]);
+}
+
+// n values of a per-particle field: the caller's, or zeros.
+template <class T> void upload_field(sph_handle *h, T *dst, const T *src, uint32_t n)
+{
+    if (!n) return;
+    if (src) cudaMemcpyAsync(dst, src, sizeof(T) * n, cudaMemcpyHostToDevice, h->stream);
+    else cudaMemsetAsync(dst, 0, sizeof(T) * n, h->stream);
 }
 
 }  // namespace
@@ -864,31 +877,17 @@ int sph_add_particles(sph_handle *h, uint32_t n, const float *pos, const float *
     if (!h || (n && (!pos || !level))) return SPH_ERR_INVALID;
     sph_readback_wait(h);   // the current buffer may still be read back
     ensure_outputs(h);      // the particles already there keep their outputs
-    const int dim = (int)h->cfg.dim;
     uint32_t n0 = read_n(h);
     if ((uint64_t)n0 + n > h->cap) { h->err = "sph_add_particles: capacity exceeded"; return SPH_ERR_CAPACITY; }
     for (uint32_t i = 0; i < n; ++i)
         if (level[i] != 1u && level[i] != 2u) { h->err = "level must be 1 or 2"; return SPH_ERR_INVALID; }
-    std::vector<float4> p4, v4, z4(n, make_float4(0.f, 0.f, 0.f, 0.f));
-    pack4(pos, dim, n, p4, level);
-    pack4(vel, dim, n, v4, nullptr);
-    std::vector<float> zf(n, 0.0f);
-    std::vector<uint32_t> zu(n, 0u);
     const CanonPtrs &b = h->buf[h->cur];
     cudaStream_t s = h->stream;
-    cudaMemcpyAsync(b.pos + n0, p4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.vel + n0, v4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.ev + n0, z4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.acc + n0, z4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.dens + n0, zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.press + n0, zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.energy + n0, zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.surface + n0, zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.interior + n0, zu.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.scene + n0, zu.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s);
+    upload_vectors(h, n0, n, pos, vel, nullptr, nullptr, level);
+    for (float *f : {b.dens, b.press, b.energy, b.surface}) upload_field<float>(h, f + n0, nullptr, n);
+    for (uint32_t *f : {b.interior, b.scene}) upload_field<uint32_t>(h, f + n0, nullptr, n);
     cudaMemsetAsync(b.sibling + n0, 0xff, sizeof(uint32_t) * n, s);
     cudaMemsetAsync(b.pos_lo + n0, 0, sizeof(float4) * n, s);
-    cudaStreamSynchronize(s);
     write_n(h, n0 + n);
     h->n_ub = n0 + n;
     h->state_gen++;
@@ -905,31 +904,18 @@ int sph_set_state(sph_handle *h, const sph_state_view *st)
     if (st->scene && h->w.nscenes)
         for (uint32_t i = 0; i < n; ++i)
             if (st->scene[i] >= h->w.nscenes) { h->err = "sph_set_state: scene index out of range"; return SPH_ERR_RANGE; }
-    const int dim = (int)h->cfg.dim;
-    std::vector<float4> p4, v4, e4, a4;
-    pack4(st->pos, dim, n, p4, st->level);
-    pack4(st->vel, dim, n, v4, nullptr);
-    pack4(st->ev, dim, n, e4, nullptr);
-    pack4(st->acc, dim, n, a4, nullptr);
-    std::vector<float> zf(n, 0.0f);
-    std::vector<uint32_t> zu(n, 0u);
     const CanonPtrs &b = h->buf[h->cur];
     cudaStream_t s = h->stream;
-    cudaMemcpyAsync(b.pos, p4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.vel, v4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.ev, e4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.acc, a4.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.dens, st->dens ? st->dens : zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.press, st->press ? st->press : zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.energy, st->energy ? st->energy : zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.surface, st->surface ? st->surface : zf.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.interior, st->interior ? st->interior : zu.data(), sizeof(uint32_t) * n,
-                    cudaMemcpyHostToDevice, s);
-    cudaMemcpyAsync(b.scene, st->scene ? st->scene : zu.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s);
+    upload_vectors(h, 0, n, st->pos, st->vel, st->ev, st->acc, st->level);
+    upload_field<float>(h, b.dens, st->dens, n);
+    upload_field<float>(h, b.press, st->press, n);
+    upload_field<float>(h, b.energy, st->energy, n);
+    upload_field<float>(h, b.surface, st->surface, n);
+    upload_field<uint32_t>(h, b.interior, st->interior, n);
+    upload_field<uint32_t>(h, b.scene, st->scene, n);
     if (st->sibling) cudaMemcpyAsync(b.sibling, st->sibling, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, s);
     else cudaMemsetAsync(b.sibling, 0xff, sizeof(uint32_t) * (n ? n : 1), s);
     cudaMemsetAsync(b.pos_lo, 0, sizeof(float4) * (n ? n : 1), s);
-    cudaStreamSynchronize(s);
     write_n(h, n);
     h->n_ub = n;
     h->have_step = false;
@@ -1291,14 +1277,17 @@ int sph_read_particles(sph_handle *h, void *host_dst, uint64_t capacity_bytes, u
     if (!h || !n_out) return SPH_ERR_INVALID;
     if (int rc = ensure_aos(h)) return rc;
     ensure_outputs(h);
+    // the conversion runs over the device's own count while the host reads it
+    const uint32_t G = grid_for(h, h->n_ub);
+    if (host_dst) {
+        if (h->cfg.dim == 3) launch(h, k_to_aos<3>, G, kThreads, 0, 0, h->cnt + h->cur, h->buf[h->cur], h->aos);
+        else launch(h, k_to_aos<2>, G, kThreads, 0, 0, h->cnt + h->cur, h->buf[h->cur], h->aos);
+    }
     const uint32_t n = read_n(h);
     const uint64_t rec = sph_particle_record_size(h);
     *n_out = n;
     if (!host_dst) return SPH_OK;
     if (capacity_bytes < rec * n) { h->err = "sph_read_particles: destination too small"; return SPH_ERR_INVALID; }
-    const uint32_t G = grid_for(h, n);
-    if (h->cfg.dim == 3) launch(h, k_to_aos<3>, G, kThreads, 0, 0, h->cnt + h->cur, h->buf[h->cur], h->aos);
-    else launch(h, k_to_aos<2>, G, kThreads, 0, 0, h->cnt + h->cur, h->buf[h->cur], h->aos);
     cudaMemcpyAsync(host_dst, h->aos, rec * n, cudaMemcpyDeviceToHost, h->stream);
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) { h->err = cudaGetErrorString(e); return SPH_ERR_CUDA; }

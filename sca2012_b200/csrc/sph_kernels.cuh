@@ -1735,6 +1735,45 @@ __global__ void __launch_bounds__(kThreads) k_from_aos(uint32_t n, CanonPtrs st,
     }
 }
 
+// ------------------------------------------------------------ state upload
+// Particles first .. first + n of a state from the caller's arrays as uploaded
+// (DIM floats per vector, null: zeros).
+struct RawState {
+    const float *pos, *vel, *ev, *acc;
+    const uint32_t *level;
+};
+
+template <int DIM>
+__global__ void __launch_bounds__(kThreads) k_unpack_state(uint32_t n, uint32_t first, RawState raw, CanonPtrs st)
+{
+    dependent_entry();
+    auto vec = [](const float *a, uint32_t i, float w) {
+        if (!a) return make_float4(0.f, 0.f, 0.f, w);
+        a += (size_t)i * DIM;
+        return make_float4(a[0], a[1], DIM == 3 ? a[2] : 0.f, w);
+    };
+    for (uint32_t i = grid_stride_start(); i < n; i += grid_stride()) {
+        const uint32_t o = first + i;
+        st.pos[o] = vec(raw.pos, i, (float)raw.level[i]);
+        st.vel[o] = vec(raw.vel, i, 0.f);
+        st.ev[o] = vec(raw.ev, i, 0.f);
+        st.acc[o] = vec(raw.acc, i, 0.f);
+    }
+}
+
+// The count of a state the host has put in place.  A new state lets steps run
+// again after a timeout, and both barrier states of the persistent step start
+// clean (a timeout leaves its abort flag set): `words` u32 from gsync on.
+__global__ void k_set_count(Counters *cnt, uint32_t n, uint32_t *gsync, uint32_t words)
+{
+    dependent_entry();
+    if (threadIdx.x == 0) {
+        cnt->n = n;
+        cnt->error &= ~(1u << SPH_ERR_TIMEOUT);
+    }
+    if (threadIdx.x < words) gsync[threadIdx.x] = 0u;
+}
+
 // ------------------------------------------------------------ conserved quantities
 // Per-block FP64 partial sums of mass, momentum (3), kinetic energy and
 // gravitational potential energy (-m g.x) over the canonical state; a second
