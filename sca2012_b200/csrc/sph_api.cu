@@ -789,6 +789,7 @@ int sph_create(const sph_config *cfg, sph_handle **out)
     w.mvs = nullptr;
     w.wall = nullptr;
     w.step_counts = nullptr;
+    w.skip_energy = 0;
     rc |= dalloc(h, &w.split_c, cap); rc |= dalloc(h, &w.removed_c, cap);
     rc |= dalloc(h, &w.split_rank, cap); rc |= dalloc(h, &w.removed_rank, cap);
     rc |= dalloc(h, &w.split_list, cap); rc |= dalloc(h, &w.leader, cap);

@@ -103,6 +103,7 @@ struct WorkPtrs {
     float *mvs;                          // taped steps only: leader slot -> summed member volume
     uint32_t *wall;                      // taped steps only: wall contacts per slot
     StepCounts *step_counts;             // taped steps only: where the write-out leaves the step's counts
+    uint32_t skip_energy;                // taped steps only: nothing reads this step's energy
     float4 *spos_lo, *spos_lo_n;         // low position parts per slot (compensated positions)
     uint32_t pos_comp;                   // the config's compensated_positions
     uint32_t *nlist, *ncnt;              // neighbour candidates (layout: nl_at), by the density pass
@@ -1109,9 +1110,10 @@ __device__ __forceinline__ void energy_split_body(const sph_config &c, Counters 
         // the density pass's candidates when the particle kept its cell and the
         // step's moves fit the margin; the stencil walk otherwise
         // (every test is false for a NaN distance or budget: such a lane walks)
+        // (no pairs at all in a taped step whose decisions do not read the energy)
         uint32_t ne = 0;
-        bool walk = valid;
-        if (valid && own_budget >= 0.0f) {
+        bool walk = valid && !w.skip_energy;
+        if (walk && own_budget >= 0.0f) {
             float ddx, ddy, ddz;
             const float d2 = r2_of<DIM>(pi, w.spos[s], ddx, ddy, ddz);
             const uint32_t cand = w.ncnt[s];
