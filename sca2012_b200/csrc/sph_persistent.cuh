@@ -212,7 +212,7 @@ __device__ __forceinline__ bool step_stages(const sph_config &c, Counters *cin, 
     // no stage reads the counts after the scan: clear them for the next hash
     for (uint32_t q = grid_stride_start(); q < a.ncells; q += grid_stride()) w.cell_count[q] = 0u;
     if (!grid_barrier(a, ++k, cin, cout)) return false;
-    reorder_body(cin, in, w);
+    reorder_body<true>(cin, in, w);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
     density_body<DIM, BS, kDensCapPersist, 8>(c, cin, w, dens);
     if (!grid_barrier(a, ++k, cin, cout)) return false;
