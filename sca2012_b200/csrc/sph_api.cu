@@ -344,11 +344,14 @@ void scan_u32(sph_handle *h, uint32_t *in, uint32_t *out, const uint32_t *len_pt
 void run_mc(sph_handle *h)
 {
     McBuffers &mc = h->mc;
-    // one thread per cube: every thread's corner loads are in flight at once
-    const uint32_t GQ = (mc.cubes + kThreads - 1) / kThreads;
-    launch(h, k_mc_count, GQ, kThreads, 0, 0, h->cfg, mc.dens, mc.cube_cnt);
+    // the longest walks in y that leave four blocks per SM
+    const uint32_t *nd = h->cfg.ndens;
+    const uint32_t tx = (nd[0] + kMcTile - 2) / kMcTile, tz = (nd[2] + kMcTile - 2) / kMcTile, Cm = nd[1] - 1;
+    const uint32_t segs = std::min(Cm, std::max((Cm + 15u) / 16u, (uint32_t)(4 * h->num_sms) / (tx * tz)));
+    const uint32_t ys = (Cm + segs - 1) / segs;
+    launch(h, k_mc_count, tx * tz * ((Cm + ys - 1) / ys), kThreads, 0, 0, h->cfg, mc.dens, mc.cube_cnt, ys);
     scan_u32(h, mc.cube_cnt, mc.cube_off, nullptr, mc.cubes, mc.num_tri, 0, nullptr);
-    launch(h, k_mc_emit, GQ, kThreads, 0, 0, h->cfg, mc.dens, mc.normal, mc.cube_cnt, mc.cube_off, mc.max_tri, mc.tri);
+    launch(h, k_mc_emit, (mc.cubes + kThreads - 1) / kThreads, kThreads, 0, 0, h->cfg, mc.dens, mc.normal, mc.cube_cnt, mc.cube_off, mc.max_tri, mc.tri);
     h->last_launches += 2;
 }
 
@@ -459,9 +462,9 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
     // density grid + surface mid-step: stale cell lists, integrated positions
     // (SPH-3D-2/sph_system.cpp:336-362)
     if (DIM == 3 && c.grid_every && h->mc.nodes && h->step_index % c.grid_every == 0) {
-        // one thread per node pair, uncapped: the block scheduler spreads the
-        // heavy pairs (cells of split particles hold four times the candidates)
-        launch_pairs(h, k_splat, (h->mc.nodes / 2 + kThreads) / kThreads, kThreads, 0, c, w.cell_off, w.spos_n, h->mc.dens);
+        // one thread per 2 x 2 nodes, uncapped: the block scheduler spreads the
+        // heavy ones (cells of split particles hold four times the candidates)
+        launch_pairs(h, k_splat, (splat_groups(c.ndens) + kSplatThreads - 1) / kSplatThreads, kSplatThreads, 0, c, w.cell_off, w.spos_n, h->mc.dens);
         launch(h, k_grid_normals, (h->mc.nodes + kThreads - 1) / kThreads, kThreads, 0, 0, c, h->mc.dens, h->mc.normal);
         h->last_launches += 2;
         run_mc(h);

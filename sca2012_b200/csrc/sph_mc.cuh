@@ -57,18 +57,32 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // weight is m * poly6(R) * (R^2 - r^2)^3 with R the particle radius, or the
 // kernel length when splat_with_kernel is set.
 //
-// One thread per pair of x-adjacent nodes (2m-1, 2m): with two nodes per cell
-// edge both usually map to the same cell, so each candidate is loaded once
-// for two nodes.  Each node still sums exactly its own stencil's particles in
-// its own walk order (a node whose cell differs from its partner's takes the
+// One thread per 2 x 2 nodes, (2m-1, 2m) in x and in y: with two or more nodes
+// per cell edge all four usually map to the same cell, so each candidate is
+// loaded once for four nodes.  Each node still sums exactly its own stencil's
+// particles in its own walk order.  Four nodes of more than one cell are
+// taken as two x pairs (a node whose cell differs from its partner's takes the
 // candidates of the joint row range that fall in its own range).
-__global__ void __launch_bounds__(kThreads) k_splat(sph_config c, const uint32_t *off,
+//
+// Bound by the candidates' loads (lanes of a warp read different cells, so a
+// 16-byte load is many L1 requests) and by issue: four nodes per load instead
+// of two took 1.24M particles on 8.5M nodes from 414 to 223 us with 256-thread
+// blocks; with 128 the heavy groups spread better (surface stage 29.3 -> 28.1
+// us a step, built every tenth).
+constexpr uint32_t kSplatThreads = 128;
+
+__host__ __device__ inline uint32_t splat_groups(const uint32_t *ndens)
+{
+    return (ndens[0] / 2 + 1) * (ndens[1] / 2 + 1) * ndens[2];   // groups {0}, {1, 2}, {3, 4}, ... in x and y
+}
+
+__global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uint32_t *off,
                                                    const float4 *pos, float *dens)
 {
     dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
-    const uint32_t GX = R / 2 + 1;   // groups {0}, {1, 2}, {3, 4}, ...
-    const uint32_t G = GX * Cn * L;
+    const uint32_t GX = R / 2 + 1, GY = Cn / 2 + 1;
+    const uint32_t G = splat_groups(c.ndens);
     // per level: the squared splat radius and m * W's coefficient
     const float rad0 = c.splat_with_kernel ? c.kernel[0] : c.radius[0];
     const float rad1 = c.splat_with_kernel ? c.kernel[1] : c.radius[1];
@@ -76,62 +90,84 @@ __global__ void __launch_bounds__(kThreads) k_splat(sph_config c, const uint32_t
     const float cf0 = __fmul_rn(c.mass[0], c.splat_with_kernel ? c.poly6[0] : c.poly6_radius[0]);
     const float cf1 = __fmul_rn(c.mass[1], c.splat_with_kernel ? c.poly6[1] : c.poly6_radius[1]);
     for (uint32_t g = grid_stride_start(); g < G; g += grid_stride()) {
-        const uint32_t gx = g % GX, vy = (g / GX) % Cn, vz = g / (GX * Cn);
-        const size_t row = ((size_t)vz * Cn + vy) * R;
+        const uint32_t gx = g % GX, gyz = g / GX, gy = gyz % GY, vz = gyz / GY;
         const uint32_t va = 2u * gx - 1u, vb = 2u * gx;   // va is not a node when gx = 0
-        const bool has_b = vb < R;
-        if (gx == 0 || vy == 0 || vz == 0) {
-            if (gx > 0) dens[row + va] = 0.0f;
-            if (has_b) dens[row + vb] = 0.0f;
+        const uint32_t ya = 2u * gy - 1u, yb = 2u * gy;   // ya is not a node when gy = 0
+        const bool has_b = vb < R, has_yb = yb < Cn;
+        float *const row_a = dens + ((size_t)vz * Cn + ya) * R, *const row_b = dens + ((size_t)vz * Cn + yb) * R;
+        if (gx == 0 || gy == 0 || vz == 0) {
+            if (gy > 0) {
+                if (gx > 0) row_a[va] = 0.0f;
+                if (has_b) row_a[vb] = 0.0f;
+            }
+            if (has_yb) {   // row 0 is a face; above it only the nodes of a face
+                if (gx > 0) row_b[va] = 0.0f;
+                if (has_b) row_b[vb] = 0.0f;
+            }
             continue;
         }
-        auto cell_x = [&](uint32_t vx) {
-            return min((uint32_t)floorf(__fmul_rn(__fdiv_rn((float)vx, (float)R), (float)c.ncell[0])),
-                       c.ncell[0] - 1);
+        auto cell = [&](uint32_t v, int a) {
+            return min((uint32_t)floorf(__fmul_rn(__fdiv_rn((float)v, (float)c.ndens[a]), (float)c.ncell[a])),
+                       c.ncell[a] - 1);
         };
-        uint3 q;
-        q.x = cell_x(va);
-        q.y = (uint32_t)floorf(__fmul_rn(__fdiv_rn((float)vy, (float)Cn), (float)c.ncell[1]));
-        q.z = (uint32_t)floorf(__fmul_rn(__fdiv_rn((float)vz, (float)L), (float)c.ncell[2]));
-        q.y = min(q.y, c.ncell[1] - 1); q.z = min(q.z, c.ncell[2] - 1);
-        const uint32_t qbx = has_b ? cell_x(vb) : q.x;
-        const float ny = __fmul_rn((float)vy, c.den_size), nz = __fmul_rn((float)vz, c.den_size);
-        const float4 npa = make_float4(__fmul_rn((float)va, c.den_size), ny, nz, 0.f);
-        const float4 npb = make_float4(__fmul_rn((float)vb, c.den_size), ny, nz, 0.f);
-        float acc_a = 0.0f, acc_b = 0.0f;
+        const uint32_t qax = cell(va, 0), qbx = has_b ? cell(vb, 0) : qax;
+        const uint32_t qya = cell(ya, 1), qyb = has_yb ? cell(yb, 1) : qya, qz = cell(vz, 2);
+        const float xa = __fmul_rn((float)va, c.den_size), xb = __fmul_rn((float)vb, c.den_size);
+        const float nya = __fmul_rn((float)ya, c.den_size), nyb = __fmul_rn((float)yb, c.den_size);
+        const float nz = __fmul_rn((float)vz, c.den_size);
         // acc += (m * W) * (rad^2 - r^2)^3 over r^2 < rad^2
-        auto add = [&](float &acc, const float4 &np, const float4 &pj, bool l1) {
+        auto add = [&](float &acc, float nx, float ny, const float4 &pj, bool l1) {
             float dx, dyy, dzz;
-            const float r2 = r2_of<3>(pj, np, dx, dyy, dzz);
+            const float r2 = r2_of<3>(pj, make_float4(nx, ny, nz, 0.f), dx, dyy, dzz);
             const float rad2 = l1 ? rs0 : rs1;
             const float x = __fsub_rn(rad2, r2);
             if (r2 < rad2) acc = __fmaf_rn(l1 ? cf0 : cf1, __fmul_rn(__fmul_rn(x, x), x), acc);
         };
-        const uint3 qb = make_uint3(qbx, q.y, q.z);
-        for (int dz = -1; dz <= 1; ++dz)
-            for (int dy = -1; dy <= 1; ++dy) {
-                uint32_t ba, ea;
-                if (!row_range<3>(c, off, q, dy, dz, ba, ea)) continue;
-                if (qbx == q.x) {   // one stencil for both nodes
-                    for (uint32_t t = ba; t < ea; ++t) {
+        if (qbx == qax && qyb == qya) {   // one stencil for all four
+            const uint3 q = make_uint3(qax, qya, qz);
+            float aa = 0.0f, ba = 0.0f, ab = 0.0f, bb = 0.0f;
+            for (int dz = -1; dz <= 1; ++dz)
+                for (int dy = -1; dy <= 1; ++dy) {
+                    uint32_t b, e;
+                    if (!row_range<3>(c, off, q, dy, dz, b, e)) continue;
+                    for (uint32_t t = b; t < e; ++t) {
                         const float4 pj = pos[t];
                         const bool l1 = pj.w == 1.0f;
-                        add(acc_a, npa, pj, l1);
-                        add(acc_b, npb, pj, l1);
+                        add(aa, xa, nya, pj, l1);
+                        add(ba, xb, nya, pj, l1);
+                        add(ab, xa, nyb, pj, l1);
+                        add(bb, xb, nyb, pj, l1);
                     }
-                } else {   // node b's row range starts and ends later in slot order
-                    uint32_t bb, eb;
+                }
+            row_a[va] = aa;
+            if (has_b) row_a[vb] = ba;
+            if (has_yb) {
+                row_b[va] = ab;
+                if (has_b) row_b[vb] = bb;
+            }
+            continue;
+        }
+        for (int yi = 0; yi < (has_yb ? 2 : 1); ++yi) {
+            const float ny = yi ? nyb : nya;
+            const uint3 qa = make_uint3(qax, yi ? qyb : qya, qz), qb = make_uint3(qbx, qa.y, qz);
+            float acc_a = 0.0f, acc_b = 0.0f;
+            for (int dz = -1; dz <= 1; ++dz)
+                for (int dy = -1; dy <= 1; ++dy) {
+                    uint32_t ba, ea, bb, eb;
+                    if (!row_range<3>(c, off, qa, dy, dz, ba, ea)) continue;
+                    // node b's row range starts and ends later in slot order, or is the same
                     row_range<3>(c, off, qb, dy, dz, bb, eb);
                     for (uint32_t t = ba; t < eb; ++t) {
                         const float4 pj = pos[t];
                         const bool l1 = pj.w == 1.0f;
-                        if (t < ea) add(acc_a, npa, pj, l1);
-                        if (t >= bb) add(acc_b, npb, pj, l1);
+                        if (t < ea) add(acc_a, xa, ny, pj, l1);
+                        if (t >= bb) add(acc_b, xb, ny, pj, l1);
                     }
                 }
-            }
-        dens[row + va] = acc_a;
-        if (has_b) dens[row + vb] = acc_b;
+            float *const row = yi ? row_b : row_a;
+            row[va] = acc_a;
+            if (has_b) row[vb] = acc_b;
+        }
     }
 }
 
@@ -142,15 +178,24 @@ __global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const f
     const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
     const uint32_t G = R * Cn * L;
     for (uint32_t g = grid_stride_start(); g < G; g += grid_stride()) {
-        const uint32_t v[3] = {g % (R * Cn) % R, g % (R * Cn) / R, g / (R * Cn)};
+        const uint32_t yz = g / R, vz = yz / Cn;
+        const uint32_t v[3] = {g - yz * R, yz - vz * Cn, vz};
         const uint32_t dims[3] = {R, Cn, L};
         const uint32_t stride[3] = {1u, R, R * Cn};
         float n[3];
         for (int a = 0; a < 3; ++a) {
             const float lo = v[a] == 0 ? 0.0f : dens[g - stride[a]];
             const float hi = v[a] == dims[a] - 1 ? 0.0f : dens[g + stride[a]];
-            n[a] = (lo - hi) / c.den_size;
+            n[a] = lo - hi;
         }
+        // no gradient (all of the empty space): what the divisions below give,
+        // without their instructions, which bound this kernel (1.24M-particle
+        // scene 38 -> 24 us)
+        if (n[0] == 0.0f && n[1] == 0.0f && n[2] == 0.0f && c.den_size > 0.0f) {
+            normal[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+            continue;
+        }
+        for (int a = 0; a < 3; ++a) n[a] /= c.den_size;
         const float len = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
         normal[g] = len == 0.0f ? make_float4(0.f, 0.f, 0.f, 0.f)
                                 : make_float4(n[0] / len, n[1] / len, n[2] / len, 0.f);
@@ -158,14 +203,13 @@ __global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const f
 }
 
 __device__ __forceinline__ uint32_t mc_cube_case(const sph_config &c, const float *dens, uint32_t x,
-                                                 uint32_t y, uint32_t z, uint32_t *corner_node)
+                                                 uint32_t y, uint32_t z)
 {
     const uint32_t R = c.ndens[0], Cn = c.ndens[1];
     uint32_t flags = 0;
     for (int v = 0; v < 8; ++v) {
         const uint32_t g = (z + kMcCornerOffset[v][2]) * R * Cn + (y + kMcCornerOffset[v][1]) * R +
                            (x + kMcCornerOffset[v][0]);
-        corner_node[v] = g;
         if (dens[g] > c.iso_value) flags |= 1u << v;   // SPH-3D-2/sph_system.cpp:459-466
     }
     return flags;
@@ -173,21 +217,59 @@ __device__ __forceinline__ uint32_t mc_cube_case(const sph_config &c, const floa
 
 __device__ __forceinline__ uint32_t mc_tri_count(uint32_t flags)
 {
-    uint32_t k = 0;
-    while (k < 5 && kMcTriangles[flags][3 * k] >= 0) ++k;
+    uint32_t k = 0;   // triangles fill a row from its start
+#pragma unroll
+    for (int j = 0; j < 5; ++j) k += kMcTriangles[flags][3 * j] >= 0;
     return k;
 }
 
+// Triangle counts.  Cubes are numbered z-innermost, nodes x-innermost: a block
+// takes 32 x 32 cubes in x and z and walks ys cubes in y, reads each plane of
+// nodes along x, keeps one byte per node of two planes in shared memory, and
+// writes the counts along z (a thread per cube read eight scattered lines for
+// its corners: 1.24M-particle scene 41.5 -> 15.5 us, 0.5M cubes 9.7 -> 5.0 us).
+constexpr uint32_t kMcTile = 32, kMcSide = kMcTile + 1, kMcPitch = 36;   // a column's bytes: 9 words apart, no bank twice
+
 __global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float *dens,
-                                                      uint32_t *cnt)
+                                                      uint32_t *cnt, uint32_t ys)
 {
+    __shared__ uint8_t in[2][kMcSide * kMcPitch], tris[256];
     dependent_entry();
-    const uint32_t Cm = c.ndens[1] - 1, Lm = c.ndens[2] - 1;
-    const uint32_t Q = (c.ndens[0] - 1) * Cm * Lm;
-    for (uint32_t q = grid_stride_start(); q < Q; q += grid_stride()) {
-        const uint32_t z = q % Lm, y = (q / Lm) % Cm, x = q / (Lm * Cm);
-        uint32_t nodes[8];
-        cnt[q] = mc_tri_count(mc_cube_case(c, dens, x, y, z, nodes));
+    const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
+    const uint32_t Rm = R - 1, Cm = Cn - 1, Lm = L - 1;
+    const uint32_t tx = (Rm + kMcTile - 1) / kMcTile, tz = (Lm + kMcTile - 1) / kMcTile;
+    const uint32_t bx = blockIdx.x % tx, bzy = blockIdx.x / tx, bz = bzy % tz;   // tiles in x, z, then runs in y
+    const uint32_t x0 = bx * kMcTile, z0 = bz * kMcTile;
+    const uint32_t y0 = (bzy / tz) * ys, y1 = min(y0 + ys, Cm);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    static_assert(kThreads == 256, "a thread per case, 8 columns of cubes per round");
+    tris[tid] = (uint8_t)mc_tri_count(tid);
+    // this thread's nodes of a plane: an offset from the plane's first node, or none
+    constexpr uint32_t kPer = (kMcSide * kMcSide + kThreads - 1) / kThreads;
+    uint32_t node[kPer], at[kPer], b[kPer];
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
+        const uint32_t u = tid + i * kThreads, zz = u / kMcSide, xx = u - zz * kMcSide;
+        at[i] = zz * kMcPitch + xx;
+        node[i] = u < kMcSide * kMcSide && x0 + xx < R && z0 + zz < L ? (z0 + zz) * Cn * R + x0 + xx : ~0u;
+        b[i] = node[i] != ~0u && dens[node[i] + y0 * R] > c.iso_value ? 2u : 0u;   // SPH-3D-2/sph_system.cpp:459-466
+    }
+    for (uint32_t y = y0; y < y1; ++y) {
+        uint8_t *const buf = in[y & 1];
+#pragma unroll
+        for (uint32_t i = 0; i < kPer; ++i) {   // bit 0: the node at y, bit 1: at y + 1
+            b[i] = (b[i] >> 1) | (node[i] != ~0u && dens[node[i] + (y + 1) * R] > c.iso_value ? 2u : 0u);
+            if (i < kPer - 1 || tid + i * kThreads < kMcSide * kMcSide) buf[at[i]] = (uint8_t)b[i];
+        }
+        __syncthreads();   // the next plane goes to the other buffer
+        if (z0 + lane < Lm) {
+            auto face = [](uint32_t lo, uint32_t hi) { return (lo & 1u) | (hi << 1) | ((lo & 2u) << 2); };
+            for (uint32_t xx = warp; xx < kMcTile && x0 + xx < Rm; xx += kThreads / 32) {
+                const uint8_t *const p = buf + lane * kMcPitch + xx;
+                const uint32_t flags = face(p[0], p[1]) | (face(p[kMcPitch], p[kMcPitch + 1]) << 4);
+                cnt[((x0 + xx) * Cm + y) * Lm + z0 + lane] = tris[flags];
+            }
+        }
     }
 }
 
@@ -196,55 +278,75 @@ __global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float
 // places them (SPH-3D-2/sph_system.cpp:479-480), or linear interpolation at
 // the iso value when mc_interpolate is set; vertex normals are the mean of
 // the two node normals.
+//
+// Most cubes have none.  A block's cubes write their triangles' cases to shared
+// memory at the scanned offsets; its threads then take one vertex each, so the
+// work is even and neighbouring threads write neighbouring vertices.  (With
+// 512 or 1,024 cubes a block too few blocks are left on the surface: the
+// surface stage of 0.5M cubes 53 -> 59 and 70 us.)
 __global__ void __launch_bounds__(kThreads) k_mc_emit(sph_config c, const float *dens,
                                                      const float4 *normal,
                                                      const uint32_t *cnt,
                                                      const uint32_t *off, uint32_t max_tri,
                                                      float *tri)
 {
+    __shared__ uint32_t list[5 * kThreads];   // per triangle: cube of this block << 16 | which of its own << 8 | its case
+    __shared__ uint32_t nlist;
     dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1];
     const uint32_t Cm = Cn - 1, Lm = c.ndens[2] - 1;
     const uint32_t Q = (R - 1) * Cm * Lm;
-    float *v0 = tri, *v1 = tri + 3ull * max_tri, *v2 = tri + 6ull * max_tri;
-    float *n0 = tri + 9ull * max_tri, *n1 = tri + 12ull * max_tri, *n2 = tri + 15ull * max_tri;
-    for (uint32_t q = grid_stride_start(); q < Q; q += grid_stride()) {
-        if (cnt[q] == 0) continue;
-        const uint32_t z = q % Lm, y = (q / Lm) % Cm, x = q / (Lm * Cm);
-        uint32_t node[8];
-        const uint32_t flags = mc_cube_case(c, dens, x, y, z, node);
-        const uint32_t base = off[q];
-        for (uint32_t k = 0; k < 5; ++k) {
-            if (kMcTriangles[flags][3 * k] < 0) break;
-            const uint32_t t = base + k;
-            if (t >= max_tri) break;
-            float *vo[3] = {v0, v1, v2}, *no[3] = {n0, n1, n2};
-            for (int j = 0; j < 3; ++j) {
-                const int e = kMcTriangles[flags][3 * k + j];
-                const int a = kMcEdgeCorner[e][0], b = kMcEdgeCorner[e][1];
-                const uint32_t ga = node[a], gb = node[b];
-                float pa[3] = {__fmul_rn((float)(x + kMcCornerOffset[a][0]), c.den_size),
-                               __fmul_rn((float)(y + kMcCornerOffset[a][1]), c.den_size),
-                               __fmul_rn((float)(z + kMcCornerOffset[a][2]), c.den_size)};
-                float pb[3] = {__fmul_rn((float)(x + kMcCornerOffset[b][0]), c.den_size),
-                               __fmul_rn((float)(y + kMcCornerOffset[b][1]), c.den_size),
-                               __fmul_rn((float)(z + kMcCornerOffset[b][2]), c.den_size)};
-                const float4 na = normal[ga], nb = normal[gb];
-                float p[3];
-                if (c.mc_interpolate) {
-                    const float da = dens[ga], db = dens[gb];
-                    const float s = db != da ? (c.iso_value - da) / (db - da) : 0.5f;
-                    for (int d = 0; d < 3; ++d) p[d] = pa[d] + s * (pb[d] - pa[d]);
-                } else {
-                    for (int d = 0; d < 3; ++d) p[d] = __fdiv_rn(__fadd_rn(pa[d], pb[d]), 2.0f);
-                }
-                const float nrm[3] = {__fdiv_rn(__fadd_rn(na.x, nb.x), 2.0f), __fdiv_rn(__fadd_rn(na.y, nb.y), 2.0f),
-                                      __fdiv_rn(__fadd_rn(na.z, nb.z), 2.0f)};
-                for (int d = 0; d < 3; ++d) {
-                    vo[j][3ull * t + d] = p[d];
-                    no[j][3ull * t + d] = nrm[d];
-                }
-            }
+    auto cube_at = [&](uint32_t q, uint32_t &x, uint32_t &y, uint32_t &z) {
+        const uint32_t xy = q / Lm;
+        z = q - xy * Lm; x = xy / Cm; y = xy - x * Cm;
+    };
+    const uint32_t q0 = blockIdx.x * kThreads, q = q0 + threadIdx.x;
+    const uint32_t first = off[q0];
+    if (q < Q) {
+        const uint32_t n = cnt[q], at = off[q] - first;
+        if (n) {
+            uint32_t x, y, z;
+            cube_at(q, x, y, z);
+            const uint32_t e = (threadIdx.x << 16) | mc_cube_case(c, dens, x, y, z);
+            for (uint32_t k = 0; k < n; ++k) list[at + k] = e | (k << 8);
+        }
+        if (threadIdx.x == kThreads - 1 || q == Q - 1) nlist = at + n;
+    }
+    __syncthreads();
+    const uint32_t total = 3 * nlist;
+    for (uint32_t i = threadIdx.x; i < total; i += kThreads) {
+        const uint32_t l = i / 3, j = i - 3 * l, t = first + l;
+        if (t >= max_tri) break;
+        const uint32_t u = list[l] >> 16, k = (list[l] >> 8) & 0xffu, flags = list[l] & 0xffu;
+        uint32_t x, y, z;
+        cube_at(q0 + u, x, y, z);
+        auto corner = [&](int v) {
+            return ((z + kMcCornerOffset[v][2]) * Cn + (y + kMcCornerOffset[v][1])) * R + x + kMcCornerOffset[v][0];
+        };
+        const int e = kMcTriangles[flags][3 * k + j];
+        const int a = kMcEdgeCorner[e][0], b = kMcEdgeCorner[e][1];
+        const uint32_t ga = corner(a), gb = corner(b);
+        float pa[3] = {__fmul_rn((float)(x + kMcCornerOffset[a][0]), c.den_size),
+                       __fmul_rn((float)(y + kMcCornerOffset[a][1]), c.den_size),
+                       __fmul_rn((float)(z + kMcCornerOffset[a][2]), c.den_size)};
+        float pb[3] = {__fmul_rn((float)(x + kMcCornerOffset[b][0]), c.den_size),
+                       __fmul_rn((float)(y + kMcCornerOffset[b][1]), c.den_size),
+                       __fmul_rn((float)(z + kMcCornerOffset[b][2]), c.den_size)};
+        const float4 na = normal[ga], nb = normal[gb];
+        float p[3];
+        if (c.mc_interpolate) {
+            const float da = dens[ga], db = dens[gb];
+            const float s = db != da ? (c.iso_value - da) / (db - da) : 0.5f;
+            for (int d = 0; d < 3; ++d) p[d] = pa[d] + s * (pb[d] - pa[d]);
+        } else {
+            for (int d = 0; d < 3; ++d) p[d] = __fdiv_rn(__fadd_rn(pa[d], pb[d]), 2.0f);
+        }
+        const float nrm[3] = {__fdiv_rn(__fadd_rn(na.x, nb.x), 2.0f), __fdiv_rn(__fadd_rn(na.y, nb.y), 2.0f),
+                              __fdiv_rn(__fadd_rn(na.z, nb.z), 2.0f)};
+        float *const vo = tri + 3ull * ((size_t)j * max_tri + t), *const no = vo + 9ull * max_tri;
+        for (int d = 0; d < 3; ++d) {
+            vo[d] = p[d];
+            no[d] = nrm[d];
         }
     }
 }
