@@ -66,7 +66,7 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 //
 // Bound by the candidates' loads (lanes of a warp read different cells, so a
 // 16-byte load is many L1 requests) and by issue: four nodes per load instead
-// of two took 1.24M particles on 8.5M nodes from 414 to 223 us with 256-thread
+// of two took 1.24M particles on 3.3M nodes from 414 to 223 us with 256-thread
 // blocks; with 128 the heavy groups spread better (surface stage 29.3 -> 28.1
 // us a step, built every tenth).
 constexpr uint32_t kSplatThreads = 128;
@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(kThreads) k_grid_normals(sph_config c, const f
             n[a] = lo - hi;
         }
         // no gradient (all of the empty space): what the divisions below give,
-        // without their instructions, which bound this kernel (1.24M-particle
-        // scene 38 -> 24 us)
+        // without their instructions, which bound this kernel (3.3M nodes
+        // 38 -> 24 us)
         if (n[0] == 0.0f && n[1] == 0.0f && n[2] == 0.0f && c.den_size > 0.0f) {
             normal[g] = make_float4(0.f, 0.f, 0.f, 0.f);
             continue;
@@ -227,7 +227,7 @@ __device__ __forceinline__ uint32_t mc_tri_count(uint32_t flags)
 // takes 32 x 32 cubes in x and z and walks ys cubes in y, reads each plane of
 // nodes along x, keeps one byte per node of two planes in shared memory, and
 // writes the counts along z (a thread per cube read eight scattered lines for
-// its corners: 1.24M-particle scene 41.5 -> 15.5 us, 0.5M cubes 9.7 -> 5.0 us).
+// its corners: 3.2M cubes 41.5 -> 15.5 us, 0.5M cubes 9.7 -> 5.0 us).
 constexpr uint32_t kMcTile = 32, kMcSide = kMcTile + 1, kMcPitch = 36;   // a column's bytes: 9 words apart, no bank twice
 
 __global__ void __launch_bounds__(kThreads) k_mc_count(sph_config c, const float *dens,
