@@ -462,9 +462,12 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
     // density grid + surface mid-step: stale cell lists, integrated positions
     // (SPH-3D-2/sph_system.cpp:336-362)
     if (DIM == 3 && c.grid_every && h->mc.nodes && h->step_index % c.grid_every == 0) {
-        // one thread per 2 x 2 nodes, uncapped: the block scheduler spreads the
+        // one thread per group of nodes, uncapped: the block scheduler spreads the
         // heavy ones (cells of split particles hold four times the candidates)
-        launch_pairs(h, k_splat, (splat_groups(c.ndens) + kSplatThreads - 1) / kSplatThreads, kSplatThreads, 0, c, w.cell_off, w.spos_n, h->mc.dens);
+        const bool quads = splat_quads(c.ndens, c.ncell, h->num_sms);
+        launch_pairs(h, quads ? k_splat<true> : k_splat<false>,
+                     (splat_groups(c.ndens, quads) + kSplatThreads - 1) / kSplatThreads, kSplatThreads, 0, c, w.cell_off,
+                     w.spos_n, h->mc.dens);
         launch(h, k_grid_normals, (h->mc.nodes + kThreads - 1) / kThreads, kThreads, 0, 0, c, h->mc.dens, h->mc.normal);
         h->last_launches += 2;
         run_mc(h);

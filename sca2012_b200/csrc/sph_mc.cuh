@@ -57,12 +57,13 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // weight is m * poly6(R) * (R^2 - r^2)^3 with R the particle radius, or the
 // kernel length when splat_with_kernel is set.
 //
-// One thread per 2 x 2 nodes, (2m-1, 2m) in x and in y: with two or more nodes
-// per cell edge all four usually map to the same cell, so each candidate is
-// loaded once for four nodes.  Each node still sums exactly its own stencil's
-// particles in its own walk order.  Four nodes of more than one cell are
-// taken as two x pairs (a node whose cell differs from its partner's takes the
-// candidates of the joint row range that fall in its own range).
+// One thread per two x-adjacent nodes (2m-1, 2m), or (QUAD) per 2 x 2 nodes,
+// (2m-1, 2m) in x and in y.  Nodes of one cell have one stencil: each of its
+// candidates is loaded once for all of them.  Each node still sums exactly its
+// own stencil's particles in its own walk order.  Nodes of more than one cell
+// are taken as x pairs, row after row (a node whose cell differs from its
+// partner's takes the candidates of the joint row range that fall in its own
+// range).
 //
 // Bound by the candidates' loads (lanes of a warp read different cells, so a
 // 16-byte load is many L1 requests) and by issue: four nodes per load instead
@@ -71,18 +72,31 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // us a step, built every tenth).
 constexpr uint32_t kSplatThreads = 128;
 
-__host__ __device__ inline uint32_t splat_groups(const uint32_t *ndens)
+// 2 x 2 nodes a thread where every group lies in one cell (an even number of
+// node spacings per cell in x and y; with 1, 3 or 5 the groups that straddle
+// cells run two rows in turn: 65 x 33 x 33 nodes 59 us with x pairs, 108 with
+// groups) and five blocks per SM are left (surface stage, x pairs / groups:
+// 2 spacings, 0.1M nodes 37 / 47 us, 0.3M 57 / 53, 0.8M 107 / 78; 4 spacings,
+// 0.3M 45 / 51, 0.8M 76 / 70, 6.4M 315 / 243).
+inline bool splat_quads(const uint32_t *ndens, const uint32_t *ncell, int num_sms)
 {
-    return (ndens[0] / 2 + 1) * (ndens[1] / 2 + 1) * ndens[2];   // groups {0}, {1, 2}, {3, 4}, ... in x and y
+    return (ndens[0] - 1) % (2 * ncell[0]) == 0 && (ndens[1] - 1) % (2 * ncell[1]) == 0 &&
+           (uint64_t)ndens[0] * ndens[1] * ndens[2] >= 4ull * 5 * kSplatThreads * num_sms;
 }
 
+__host__ __device__ inline uint32_t splat_groups(const uint32_t *ndens, bool quads)
+{
+    return (ndens[0] / 2 + 1) * (quads ? ndens[1] / 2 + 1 : ndens[1]) * ndens[2];   // groups {0}, {1, 2}, {3, 4}, ...
+}
+
+template <bool QUAD>
 __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uint32_t *off,
-                                                   const float4 *pos, float *dens)
+                                                         const float4 *pos, float *dens)
 {
     dependent_entry();
     const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
-    const uint32_t GX = R / 2 + 1, GY = Cn / 2 + 1;
-    const uint32_t G = splat_groups(c.ndens);
+    const uint32_t GX = R / 2 + 1, GY = QUAD ? Cn / 2 + 1 : Cn;
+    const uint32_t G = splat_groups(c.ndens, QUAD);
     // per level: the squared splat radius and m * W's coefficient
     const float rad0 = c.splat_with_kernel ? c.kernel[0] : c.radius[0];
     const float rad1 = c.splat_with_kernel ? c.kernel[1] : c.radius[1];
@@ -92,11 +106,11 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
     for (uint32_t g = grid_stride_start(); g < G; g += grid_stride()) {
         const uint32_t gx = g % GX, gyz = g / GX, gy = gyz % GY, vz = gyz / GY;
         const uint32_t va = 2u * gx - 1u, vb = 2u * gx;   // va is not a node when gx = 0
-        const uint32_t ya = 2u * gy - 1u, yb = 2u * gy;   // ya is not a node when gy = 0
-        const bool has_b = vb < R, has_yb = yb < Cn;
+        const uint32_t ya = QUAD ? 2u * gy - 1u : gy, yb = 2u * gy;   // 2 gy - 1 is not a node when gy = 0
+        const bool has_b = vb < R, has_yb = QUAD && yb < Cn;
         float *const row_a = dens + ((size_t)vz * Cn + ya) * R, *const row_b = dens + ((size_t)vz * Cn + yb) * R;
         if (gx == 0 || gy == 0 || vz == 0) {
-            if (gy > 0) {
+            if (!QUAD || gy > 0) {
                 if (gx > 0) row_a[va] = 0.0f;
                 if (has_b) row_a[vb] = 0.0f;
             }
@@ -123,7 +137,7 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
             const float x = __fsub_rn(rad2, r2);
             if (r2 < rad2) acc = __fmaf_rn(l1 ? cf0 : cf1, __fmul_rn(__fmul_rn(x, x), x), acc);
         };
-        if (qbx == qax && qyb == qya) {   // one stencil for all four
+        if (QUAD && qbx == qax && qyb == qya) {   // one stencil for all four
             const uint3 q = make_uint3(qax, qya, qz);
             float aa = 0.0f, ba = 0.0f, ab = 0.0f, bb = 0.0f;
             for (int dz = -1; dz <= 1; ++dz)
@@ -153,9 +167,19 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
             float acc_a = 0.0f, acc_b = 0.0f;
             for (int dz = -1; dz <= 1; ++dz)
                 for (int dy = -1; dy <= 1; ++dy) {
-                    uint32_t ba, ea, bb, eb;
+                    uint32_t ba, ea;
                     if (!row_range<3>(c, off, qa, dy, dz, ba, ea)) continue;
-                    // node b's row range starts and ends later in slot order, or is the same
+                    if (qbx == qax) {   // one stencil for both
+                        for (uint32_t t = ba; t < ea; ++t) {
+                            const float4 pj = pos[t];
+                            const bool l1 = pj.w == 1.0f;
+                            add(acc_a, xa, ny, pj, l1);
+                            add(acc_b, xb, ny, pj, l1);
+                        }
+                        continue;
+                    }
+                    // node b's row range starts and ends later in slot order
+                    uint32_t bb, eb;
                     row_range<3>(c, off, qb, dy, dz, bb, eb);
                     for (uint32_t t = ba; t < eb; ++t) {
                         const float4 pj = pos[t];

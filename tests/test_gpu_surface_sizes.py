@@ -1,8 +1,9 @@
 """Node grids of odd, even and ragged sizes: the density-grid splat against the
 FP64 oracle, and marching cubes against the oracle's, cube order included.
 
-Splat: 2 x 2 node groups whose nodes share a cell (grids of k * cells + 1
-nodes) or do not (even counts), and groups cut off at the upper faces.
+Splat: 2 x 2 node groups (grids of an even multiple of the cells plus one node,
+0.4M nodes and more) and x pairs (the others), whose nodes share a cell or do
+not, and groups cut off at the upper faces.
 Marching cubes: 32 x 32 tiles and 256-cube blocks with remainders, down to a
 single cube; a random grid fills the blocks' triangle lists.
 """
@@ -33,7 +34,8 @@ def _f(a):
     return a.ctypes.data_as(C.POINTER(C.c_float))
 
 
-@pytest.mark.parametrize("dims", [(129, 65, 65), (64, 33, 20), (65, 34, 17), (130, 66, 9), (33, 17, 5), (2, 3, 2)])
+@pytest.mark.parametrize("dims", [(129, 65, 65), (64, 33, 20), (65, 34, 17), (130, 66, 9), (33, 17, 5), (2, 3, 2),
+                                  (129, 65, 60), (193, 97, 65)])
 def test_splat_matches_oracle(dims, gpu):
     cfg = _cfg(dims)
     cfg.grid_every = 1
