@@ -265,7 +265,8 @@ __global__ void __launch_bounds__(kScanThreads) scan_phase23(const T *__restrict
 // ------------------------------------------------------------ one-launch scan
 // The whole scan by ONE thread-block cluster: each warp sums its contiguous
 // segment, the blocks exchange their totals through distributed shared memory
-// and meet once at the hardware cluster barrier (nothing polls), and each warp
+// and meet at the hardware cluster barrier, before the exchange and behind it
+// (nothing polls), and each warp
 // rescans its segment, 128 elements (four per lane) at a time.  Two reads and
 // one write of the input, like the two launches above, by 16 SMs: the launch
 // and the drain between the two are saved, which is what a scan of some 100,000
@@ -292,6 +293,10 @@ __device__ __forceinline__ uint32_t cluster_scan_body(const ClusterScan &j)
 {
     __shared__ uint32_t warp_off[kClusterScanThreads / 32 + 1];
     __shared__ uint32_t block_tot[kClusterScanBlocks];
+    // A block may write another's shared memory only once that one is known to
+    // have started: each says so here, and the wait stands before the stores,
+    // behind the first read of the input.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr uint32_t nw = kClusterScanThreads / 32;
     const uint32_t nb = gridDim.x, rank = blockIdx.x;   // the grid is one cluster
@@ -316,6 +321,7 @@ __device__ __forceinline__ uint32_t cluster_scan_body(const ClusterScan &j)
     acc = __reduce_add_sync(0xffffffffu, acc);
     if (lane == 0) warp_off[warp + 1] = acc;
     __syncthreads();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");   // every block has started
     if (warp == 0) {   // exclusive offsets of the warps, block total last
         uint32_t v = warp_off[lane + 1];
         for (int d = 1; d < 32; d <<= 1) {
