@@ -557,8 +557,10 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
         };
         // whole chunks of four, then (last) the rest; up to three entries stay
         // at the front of the buffer in between
+        // (the appends in quad are opaque to the compiler: no load or store of
+        // the buffer may move across either end of the drain)
         auto drain = [&](bool last) {
-            asm volatile("" ::: "memory");   // the appends below are opaque to the compiler
+            asm volatile("" ::: "memory");
             const uint32_t fill = (at - col0) >> 8, whole = fill & ~3u;
             for (uint32_t g = 0; g < whole; g += 4) {
                 const uint2 a0 = col[(g + 0) * 32], a1 = col[(g + 1) * 32], a2 = col[(g + 2) * 32],
@@ -592,6 +594,7 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
                     if ((uint32_t)u < rest) col[u * 32] = col[(whole + u) * 32];
             }
             at = col0 + rest * 256u;
+            asm volatile("" ::: "memory");
         };
         const float2 nx = make_float2(-pi.x, -pi.x), ny = make_float2(-pi.y, -pi.y);
         // slots 2p .. 2p + 3 of the staged chunk: thr0: the bound of the first

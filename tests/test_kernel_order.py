@@ -48,3 +48,15 @@ def test_remote_shared_memory_has_one_user():
     body = _block(_code("sph_scan.cuh"), r"uint32_t\s+cluster_scan_body\(")
     assert len(re.findall(r"\bmapa\b|shared::cluster", body)) == len(
         re.findall(r"\bmapa\b|shared::cluster", _code("sph_scan.cuh")))
+
+
+def test_density_buffer_drain_is_fenced_from_the_appends():
+    """The density walk appends to its buffer by inline assembly that names no
+    memory; the drain's plain loads and stores of the same buffer stay between
+    two compiler barriers."""
+    body = _block(_code("sph_kernels.cuh"), r"void\s+density_walk\(")
+    drain = re.sub(r"\s+", "", _block(body, r"auto\s+drain\s*=\s*\[&\]\(bool\s+last\)")[1:-1])
+    fence = 'asmvolatile("":::"memory");'
+    assert drain.startswith(fence) and drain.endswith(fence)
+    # every other plain use of the buffer is inside the drain
+    assert len(re.findall(r"\bcol\[", body)) == drain.count("col[")
