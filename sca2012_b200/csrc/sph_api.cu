@@ -284,41 +284,49 @@ template <class... P, class... A> void launch_cluster(sph_handle *h, void (*kern
     h->last_launches += 1;
 }
 
-// Cluster size of the one-launch scans on a device: 16 blocks, else 8, else
-// none (0).  A property of the device, asked once per process (the occupancy
-// query takes about a millisecond).
-int query_scan_cluster(int device)
+// Cluster size of the one-launch scans on the current device: 16 blocks, else
+// 8, else none (0).  The size is a property of the device, asked once per
+// process (the occupancy query takes about a millisecond); the attribute that a
+// cluster of 16 needs belongs to the loaded module, which a cudaDeviceReset
+// unloads, so every handle sets it.
+int scan_cluster_size(int device)
 {
+    auto allow = [](int size) {
+        if (size <= 8) return true;
+        for (const void *kern : {(const void *)k_scan_cluster, (const void *)k_split_ranks})
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                return false;
+        return true;
+    };
     constexpr int kMaxDevices = 64;
     static std::atomic<int> known[kMaxDevices];   // size + 1; 0: not asked yet
-    if (device >= 0 && device < kMaxDevices) {
-        if (const int k = known[device].load()) return k - 1;
-        const int size = query_scan_cluster(-1);
-        known[device].store(size + 1);
-        return size;
-    }
-    for (int size : {kClusterScanBlocks, 8}) {
-        bool ok = true;
-        for (const void *kern : {(const void *)k_scan_cluster, (const void *)k_split_ranks}) {
-            if (size > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-                ok = false;
-            cudaLaunchConfig_t lc = {};
-            lc.gridDim = dim3(size);
-            lc.blockDim = dim3(kClusterScanThreads);
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = size;
-            attr[0].val.clusterDim.y = 1;
-            attr[0].val.clusterDim.z = 1;
-            lc.attrs = attr;
-            lc.numAttrs = 1;
-            int n = 0;
-            ok = ok && cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess && n >= 1;
+    const bool keep = device >= 0 && device < kMaxDevices;
+    int found = 0;
+    if (const int k = keep ? known[device].load() : 0) {
+        found = allow(k - 1) ? k - 1 : 0;
+    } else {
+        for (int size : {kClusterScanBlocks, 8}) {
+            bool ok = allow(size);
+            for (const void *kern : {(const void *)k_scan_cluster, (const void *)k_split_ranks}) {
+                cudaLaunchConfig_t lc = {};
+                lc.gridDim = dim3(size);
+                lc.blockDim = dim3(kClusterScanThreads);
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = size;
+                attr[0].val.clusterDim.y = 1;
+                attr[0].val.clusterDim.z = 1;
+                lc.attrs = attr;
+                lc.numAttrs = 1;
+                int n = 0;
+                ok = ok && cudaOccupancyMaxActiveClusters(&n, kern, &lc) == cudaSuccess && n >= 1;
+            }
+            if (ok) { found = size; break; }
         }
-        cudaGetLastError();
-        if (ok) return size;
+        if (keep) known[device].store(found + 1);
     }
-    return 0;
+    cudaGetLastError();   // a refused attribute or query is an answer, not an error of the next call
+    return found;
 }
 
 // Exclusive scan of u32 `in` -> `out`; length from len_ptr (device, at most
@@ -748,7 +756,7 @@ int sph_create(const sph_config *cfg, sph_handle **out)
         return SPH_ERR_CUDA;
     }
     h->own_stream = h->stream;
-    h->scan_cluster = query_scan_cluster(h->device);
+    h->scan_cluster = scan_cluster_size(h->device);
     h->cap = cfg->max_particle;
     h->ncells = total_cells(*cfg);
     const size_t cap = h->cap, C = h->ncells;
