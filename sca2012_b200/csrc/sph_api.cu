@@ -43,6 +43,7 @@ struct sph_handle {
     int scan_cluster = 0;             // blocks of a one-cluster scan (0: two launches)
     uint32_t *stat_buf = nullptr;     // sph_last_step_stats: level-2 count
     uint32_t n_ub = 0;                // host upper bound of the live count
+    uint32_t n_seen = 0;              // the live count the host last knew
     uint32_t n_last_sorted = 0;       // count the last step started with (host copy)
     bool have_step = false;
     bool debug = false;
@@ -182,11 +183,34 @@ uint32_t merge_work(const sph_handle *h)
     return (uint32_t)std::min<uint64_t>((uint64_t)h->ncells * 32u / kMergeCellsMin, 1u << 31);
 }
 
-// Launch key of the step: every stage's grid and block size (a captured
-// graph is valid while it is unchanged).
+// Whether a scan of `len` elements runs as one cluster.  16 SMs cost less than
+// the second launch (and, for the cell counts, the memset) of a full grid up to
+// about 800,000 elements: cell scan 11.0 against 15.2 us at 262,144 cells, 21.5
+// against 19.2 at 1,048,576, 59 against 34 at 4M.
+constexpr uint32_t kClusterScanMax = 3u << 18;
+
+bool scan_as_cluster(const sph_handle *h, uint32_t len) { return h->scan_cluster > 0 && len <= kClusterScanMax; }
+
+// Whether the ranks of a step's flags are scanned by one cluster.  A scan reads
+// as many elements as particles live, while the host's bound may be four times
+// that after one step: the rule goes by the count the host last knew, and the
+// bound only limits what a count grown unseen since then can cost.  Cluster
+// against full grid, split ranks with flags: 12.3 against 13.3 us at 262,144
+// particles, 18.4 / 15.4 at 589,824, 25.6 / 17.4 at 1,048,576, 71.7 / 33 at 4.2M;
+// a step without flags only checks their count, 6.1 / 9.2 at any size.  The line
+// lies where the one loses with flags what it gains without.
+constexpr uint32_t kClusterRankMax = 9u << 16, kClusterRankBound = 1u << 22;
+
+bool ranks_as_cluster(const sph_handle *h)
+{
+    return h->scan_cluster > 0 && std::min(h->n_ub, h->n_seen) <= kClusterRankMax && h->n_ub <= kClusterRankBound;
+}
+
+// Launch key of the step: every stage's grid and block size and the form of
+// its rank scans (a captured graph is valid while it is unchanged).
 uint64_t launch_key(const sph_handle *h)
 {
-    uint64_t k = 1469598103934665603ull;
+    uint64_t k = 1469598103934665603ull ^ (ranks_as_cluster(h) ? 1u : 0u);
     for (int st = 0; st < SPH_TUNE_STAGES; ++st) {
         const uint32_t work = st == SPH_TUNE_MERGE ? merge_work(h) : h->n_ub;
         k = (k ^ grid_st(h, work, st)) * 1099511628211ull;
@@ -217,20 +241,6 @@ uint64_t launch_key(const sph_handle *h)
     case 256 * 16 + 1: { constexpr int B = 256, M = 4; __VA_ARGS__; } break;            \
     default: { constexpr int B = 256, M = 3; __VA_ARGS__; } break;                      \
     }
-
-// Whether a scan of at most `bound` elements runs as one cluster.  16 SMs cost
-// less than the second launch (and, for the cell counts, the memset) of a full
-// grid up to about 800,000 elements: cell scan 11.0 against 15.2 us at 262,144
-// cells, 21.5 against 19.2 at 1,048,576, 59 against 34 at 4M.  A rank scan
-// whose flags may be all zero (most steps) only checks their count then, 6
-// against 11-13 us, which pays up to a bound of 4M (the host's bound of the
-// particle count, up to four times the count itself).
-constexpr uint32_t kClusterScanMax = 3u << 18, kClusterRankMax = 1u << 22;
-
-bool scan_as_cluster(const sph_handle *h, uint32_t bound, bool ranks)
-{
-    return h->scan_cluster > 0 && bound <= (ranks ? kClusterRankMax : kClusterScanMax);
-}
 
 // Launches a kernel that begins with dependent_entry(), dependent: as a
 // programmatic dependent of the kernel before it in the handle's stream (any
@@ -329,23 +339,42 @@ int scan_cluster_size(int device)
     return found;
 }
 
-// Exclusive scan of u32 `in` -> `out`; length from len_ptr (device, at most
-// `bound`) or bound itself.  skip_if_zero: a device count of the nonzero
-// inputs (0: only the total is written).  clear: zero the input behind the scan.
-void scan_u32(sph_handle *h, uint32_t *in, uint32_t *out, const uint32_t *len_ptr, uint32_t bound, uint32_t *grand,
-              int total_at_len, uint32_t *list, const uint32_t *skip_if_zero = nullptr, bool clear = false)
+// Exclusive scan of `len` u32, in -> out; the total to *grand and, if
+// total_at_len, to out[len].  clear: zero the input behind the scan.
+void scan_u32(sph_handle *h, uint32_t *in, uint32_t *out, uint32_t len, uint32_t *grand, int total_at_len,
+              bool clear = false)
 {
-    if (scan_as_cluster(h, bound, skip_if_zero != nullptr)) {
-        launch_cluster(h, k_scan_cluster, ClusterScan{in, out, len_ptr, bound, grand, list, skip_if_zero, total_at_len,
+    if (scan_as_cluster(h, len)) {
+        launch_cluster(h, k_scan_cluster, ClusterScan{in, out, nullptr, len, grand, nullptr, nullptr, total_at_len,
                                                       clear ? 1 : 0});
         return;
     }
-    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, len_ptr, bound, h->scan_blocks,
-                                                                       skip_if_zero);
-    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, len_ptr, bound, h->scan_blocks,
-                                                                        grand, total_at_len, list, skip_if_zero);
+    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, nullptr, len, h->scan_blocks);
+    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, nullptr, len, h->scan_blocks, grand,
+                                                                        total_at_len, nullptr);
     h->last_launches += 2;
-    if (clear) cudaMemsetAsync(in, 0, sizeof(uint32_t) * bound, h->stream);
+    if (clear) cudaMemsetAsync(in, 0, sizeof(uint32_t) * len, h->stream);
+}
+
+// Ranks of a step's split flags (with the list of split particles and the
+// capacity guard) or removal flags.
+void scan_ranks(sph_handle *h, Counters *cin, bool splits)
+{
+    const WorkPtrs &w = h->w;
+    uint32_t *const flags = splits ? w.split_c : w.removed_c, *const ranks = splits ? w.split_rank : w.removed_rank;
+    uint32_t *const list = splits ? w.split_list : nullptr, *const count = splits ? &cin->split_flags : &cin->removed_flags;
+    uint32_t *const total = splits ? &cin->n_split : &cin->n_removed;
+    if (!ranks_as_cluster(h)) {
+        const RankScan j{flags, ranks, list, h->scan_blocks, count, total, splits ? 1 : 0};
+        launch(h, k_rank_totals, kScanBlocks, kScanThreads, 0, 0, j, cin);
+        launch(h, k_ranks, kScanBlocks, kScanThreads, 0, 0, j, h->cfg, cin, h->cap);
+        h->last_launches += 2;
+    } else if (splits) {
+        launch_cluster(h, k_split_ranks, ClusterScan{flags, ranks, &cin->n, 0, nullptr, list, nullptr, 0, 0}, h->cfg, cin,
+                       h->cap);
+    } else {
+        launch_cluster(h, k_scan_cluster, ClusterScan{flags, ranks, &cin->n, 0, total, nullptr, count, 0, 0});
+    }
 }
 
 // Marching cubes over the current device grid: classify, scan, emit.
@@ -358,7 +387,7 @@ void run_mc(sph_handle *h)
     const uint32_t segs = std::min(Cm, std::max((Cm + 15u) / 16u, (uint32_t)(4 * h->num_sms) / (tx * tz)));
     const uint32_t ys = (Cm + segs - 1) / segs;
     launch(h, k_mc_count, tx * tz * ((Cm + ys - 1) / ys), kThreads, 0, 0, h->cfg, mc.dens, mc.cube_cnt, ys);
-    scan_u32(h, mc.cube_cnt, mc.cube_off, nullptr, mc.cubes, mc.num_tri, 0, nullptr);
+    scan_u32(h, mc.cube_cnt, mc.cube_off, mc.cubes, mc.num_tri, 0);
     launch(h, k_mc_emit, (mc.cubes + kThreads - 1) / kThreads, kThreads, 0, 0, h->cfg, mc.dens, mc.normal, mc.cube_cnt, mc.cube_off, mc.max_tri, mc.tri);
     h->last_launches += 2;
 }
@@ -448,7 +477,7 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
         stage(h, "hash");
     }
     // the counts are cleared behind the scan, for the write-out's hash of the next state
-    scan_u32(h, w.cell_count, w.cell_off, nullptr, h->ncells, h->scan_grand, 1, nullptr, nullptr, true);
+    scan_u32(h, w.cell_count, w.cell_off, h->ncells, h->scan_grand, 1, true);
     h->counts_zero = false;
     stage(h, "scan_cells");
     SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_SCATTER], 
@@ -488,14 +517,7 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
     stage(h, "energy_split");
     h->last_launches += 5;
     if (c.use_split) {   // else no particle is flagged
-        if (scan_as_cluster(h, nub, true)) {
-            launch_cluster(h, k_split_ranks, ClusterScan{w.split_c, w.split_rank, &cin->n, nub, nullptr, w.split_list,
-                                                         nullptr, 0, 0}, c, cin, h->cap);
-        } else {
-            scan_u32(h, w.split_c, w.split_rank, &cin->n, nub, &cin->n_split, 0, w.split_list, &cin->split_flags);
-            launch(h, k_split_guard, 1, 1, 0, 0, c, cin, h->cap);
-            h->last_launches += 1;
-        }
+        scan_ranks(h, cin, true);
         stage(h, "scan_split");
     }
     if (c.use_merge) {
@@ -504,7 +526,7 @@ template <int DIM> int run_step(sph_handle *h, bool prologue = true)
                              h->ncells, h->cap));
         h->last_launches += 1;
         stage(h, "merge");
-        scan_u32(h, w.removed_c, w.removed_rank, &cin->n, nub, &cin->n_removed, 0, nullptr, &cin->removed_flags);
+        scan_ranks(h, cin, false);
         stage(h, "scan_removed");
     }
     SPH_BS_SWITCH(h->tune_bs[SPH_TUNE_WRITE],
@@ -684,6 +706,7 @@ uint32_t read_n(sph_handle *h)
     uint32_t n = 0;
     cudaMemcpyAsync(&n, &h->cnt[h->cur].n, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream);
     cudaStreamSynchronize(h->stream);
+    h->n_seen = n;
     return n;
 }
 
@@ -697,6 +720,7 @@ void write_n(sph_handle *h, uint32_t n)
     h->counts_zero = false;      // the cell counts are cleared before the next launch
     h->counts_hashed = false;
     h->outputs_pending = false;  // the caller wrote every field
+    h->n_seen = n;
     cudaStreamSynchronize(h->stream);
 }
 
@@ -1142,6 +1166,7 @@ int sph_sync(sph_handle *h)
     if (e != cudaSuccess) { h->err = cudaGetErrorString(e); return SPH_ERR_CUDA; }
     Counters c0;
     cudaMemcpy(&c0, &h->cnt[h->cur], sizeof(Counters), cudaMemcpyDeviceToHost);
+    h->n_seen = c0.n;
     if (c0.error) {
         uint32_t err = c0.error;
         c0.error = 0;

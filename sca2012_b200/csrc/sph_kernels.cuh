@@ -1224,12 +1224,6 @@ __device__ __forceinline__ void split_guard_body(const sph_config &c, Counters *
     }
 }
 
-__global__ void k_split_guard(const sph_config c, Counters *cnt, uint32_t cap)
-{
-    dependent_entry();
-    split_guard_body(c, cnt, cnt->n_split, cap);
-}
-
 __global__ void __launch_bounds__(kClusterScanThreads) k_scan_cluster(ClusterScan j)
 {
     dependent_entry();
@@ -1249,6 +1243,36 @@ __global__ void __launch_bounds__(kClusterScanThreads) k_split_ranks(ClusterScan
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         cnt->n_split = total;
         split_guard_body(c, cnt, total, cap);
+    }
+}
+
+// The ranks of a step's flags by a full grid of kScanBlocks, where 16 SMs are
+// too few: chunk totals, then rescans.  Bound: the two reads and one write of
+// the flags and the launches; 592 and 296 blocks save 2 us where there are no
+// flags and lose 8 and 30 at 4.2M.  As ordinary launches with the guard a third
+// one: 19.5 instead of 17.4 us at 1.05M particles, 12.3 instead of 9.2 without
+// flags.  flags: their device count (at 0 only the total is written); guard:
+// the flags are splits.
+struct RankScan {
+    uint32_t *in, *out, *list, *block_tot;
+    const uint32_t *flags;
+    uint32_t *total;
+    int guard;
+};
+
+__global__ void __launch_bounds__(kScanThreads) k_rank_totals(RankScan j, const Counters *cnt)
+{
+    dependent_entry();
+    if (*j.flags) scan_phase1_body<uint32_t>(j.in, cnt->n, j.block_tot);
+}
+
+__global__ void __launch_bounds__(kScanThreads) k_ranks(RankScan j, const sph_config c, Counters *cnt, uint32_t cap)
+{
+    dependent_entry();
+    if (*j.flags) scan_phase23_body<uint32_t>(j.in, j.out, cnt->n, j.block_tot, j.total, 0, j.list);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the thread that wrote the total
+        if (*j.flags == 0u) *j.total = 0u;
+        if (j.guard) split_guard_body(c, cnt, *j.total, cap);
     }
 }
 

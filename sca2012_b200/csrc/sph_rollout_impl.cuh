@@ -110,6 +110,7 @@ int restore_ckpt(sph_handle *h, Rollout *r, size_t k)
     cudaMemcpyAsync(&h->cnt[h->cur], &c0, sizeof(Counters), cudaMemcpyHostToDevice, h->stream);
     cudaStreamSynchronize(h->stream);
     h->n_ub = n;
+    h->n_seen = n;
     h->counts_hashed = false;   // the hash a persistent step left is not this state's
     h->outputs_pending = false;
     return cuda_check(h, "rollout: restore checkpoint");
@@ -222,7 +223,7 @@ template <int DIM> void sort_only(sph_handle *h)
     h->counts_zero = false;
     h->counts_hashed = false;
     launch(h, k_hash<DIM>, G, kThreads, 0, 0, c, cin, in, w);
-    scan_u32(h, w.cell_count, w.cell_off, nullptr, h->ncells, h->scan_grand, 1, nullptr);
+    scan_u32(h, w.cell_count, w.cell_off, h->ncells, h->scan_grand, 1);
     launch(h, k_scatter<>, G, kThreads, 0, 0, cin, w);
     launch(h, k_reorder<>, G, kThreads, 0, 0, cin, in, w);
 }
@@ -317,7 +318,7 @@ template <int DIM> int topology_impl(sph_handle *h, Rollout *r, uint32_t step, s
     k_topo_pairs<DIM, false><<<G, kThreads, 0, s>>>(c, k, t, r->tcount[0], r->tcount[1], nullptr, nullptr, nullptr,
                                                      nullptr);
     for (int q = 0; q < 2; ++q)
-        scan_u32(h, r->tcount[q], r->toff[q], nullptr, n, h->scan_grand, 1, nullptr);
+        scan_u32(h, r->tcount[q], r->toff[q], n, h->scan_grand, 1);
     uint32_t tot[2];
     for (int q = 0; q < 2; ++q)
         cudaMemcpyAsync(&tot[q], r->toff[q] + n, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
