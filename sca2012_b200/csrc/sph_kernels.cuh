@@ -229,8 +229,7 @@ __device__ __forceinline__ float r2_of(float4 a, float4 b, float &dx, float &dy,
     return t;
 }
 
-// 1/sqrt(x) as rsqrtf gives it, without the rescaling of denormal x (+inf
-// there, as for 0).
+// 1/sqrt(x) by the PTX instruction, whose .ftz takes a denormal x as zero (+inf).
 __device__ __forceinline__ float rsqrt_normal(float x)
 {
     float y;
@@ -240,8 +239,8 @@ __device__ __forceinline__ float rsqrt_normal(float x)
 
 // sqrt(x) from y = rsqrt_normal(x) by one Newton step with the residual in
 // one fused multiply-add (Markstein, IBM J. Res. Dev. 34, 1990): no branch
-// and no second special-function instruction.  Compared with __fsqrt_rn over
-// every FP32 value in [2.7e-20, 4e37]: the same bits.  Not for x = 0 (NaN).
+// and no second special-function instruction.  The bits of __fsqrt_rn for every
+// FP32 value in [2.7e-20, 4e37] (compared value by value).  Not for x = 0 (NaN).
 __device__ __forceinline__ float sqrt_of(float x, float y)
 {
     const float g = __fmul_rn(x, y);
@@ -1036,8 +1035,10 @@ __global__ void __launch_bounds__(BS, MINB) k_force_integrate(sph_config c, Coun
 // 0.215 ms; 1.05M plain: 0.151 -> 0.134 ms.
 // psi(x) = amp * (x^2/4 - 1) * EXP^(-x^2/8), EXP = 2.718281f (sigma = 2), for
 // |x| < 30: x^2/4 is exact, so one fused multiply-add rounds as the difference
-// does; the exponent's factor 1/8 is an exact scaling; and the exponential is
-// exp2f's without its rescaling of results below 2^-126.
+// does; the exponent's factor 1/8 is an exact scaling.
+// 2^x by the PTX instruction, whose .ftz gives zero for a result below 2^-126;
+// the bits of exp2f for every FP32 value in [-126, 0] (compared value by value;
+// a pair inside the kernel has x >= -0.19).
 __device__ __forceinline__ float ex2_normal(float x)
 {
     float y;
