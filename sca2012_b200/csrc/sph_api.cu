@@ -219,8 +219,9 @@ uint64_t launch_key(const sph_handle *h)
     return k;
 }
 
-// Instantiates a launch for the stage's block size B (128, 256 or 512; the
-// SWITCH2 kernels hold a 48 KB shared list at 256 threads and stop at 256).
+// Instantiates a launch for the stage's block size B (128, 256 or 512).  The
+// SWITCH2 kernels stop at 256: at 80 to 96 registers an SM holds one block of
+// 512 threads, and a quarter or more of its registers stay unused.
 #define SPH_BS_SWITCH(bs, ...)                                   \
     switch (bs) {                                                \
     case 128: { constexpr int B = 128; __VA_ARGS__; } break;     \

@@ -106,7 +106,11 @@ struct WorkPtrs {
     uint32_t skip_energy;                // taped steps only: nothing reads this step's energy
     float4 *spos_lo, *spos_lo_n;         // low position parts per slot (compensated positions)
     uint32_t pos_comp;                   // the config's compensated_positions
-    uint32_t *nlist, *ncnt;              // neighbour candidates (layout: nl_at), by the density pass
+    // neighbour candidates, by the density pass.  Entries come in chunks of four
+    // (one 16-byte load); chunk j of every slot is one row of nl_stride chunks, so
+    // the chunk-j loads of a warp's 32 consecutive slots read 512 contiguous bytes:
+    // entry k of slot s is nlist[((k >> 2) * nl_stride + s) * 4 + (k & 3)].
+    uint32_t *nlist, *ncnt;
     uint32_t nl_stride;                  // slots per list chunk row (the capacity)
     float4 *fnb_a, *fnb_b;               // a force neighbour in two loads: (x, y, z, p/rho^2) and
                                          // (m/rho with the sign bit set for level 2, ev.xyz), by the density pass
@@ -143,14 +147,6 @@ constexpr float kNbrListMargin = 0.05f;
 __device__ __forceinline__ void prefetch_l2(const void *p)
 {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
-// Entry k of slot s's list.  Entries come in chunks of four (one 16-byte
-// load); chunk j of every slot is one row, so the chunk-j loads of a warp's
-// 32 consecutive slots read 512 contiguous bytes.
-__device__ __forceinline__ size_t nl_at(const WorkPtrs &w, uint32_t s, uint32_t k)
-{
-    return (size_t)(k >> 2) * ((size_t)w.nl_stride * 4u) + (size_t)s * 4u + (k & 3u);
 }
 
 __device__ __forceinline__ float energy_list_r2(const sph_config &c)
@@ -519,7 +515,7 @@ __device__ __forceinline__ void density_walk(const sph_config &c, Counters *cnt,
     // the append position as a shared-memory address (256 bytes per entry)
     const uint32_t col0 = (uint32_t)__cvta_generic_to_shared(col), col_lim = col0 + (CAP - 4) * 256u;
     constexpr int nrows = DIM == 3 ? 9 : 3, own = nrows / 2;
-    // list entry k at lbase[(k >> 2) * row4 + (k & 3)] (nl_at; the offset
+    // list entry k at lbase[(k >> 2) * row4 + (k & 3)] (the offset
     // fits 32 bits under the lists' 12 GB allocation limit)
     const bool rec = w.nlist != nullptr;
     const uint32_t row4 = w.nl_stride * 4u;

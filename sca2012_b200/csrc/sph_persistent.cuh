@@ -185,8 +185,9 @@ __device__ __forceinline__ bool grid_scan(const PersistArgs &a, uint32_t &k, Cou
 // phase (scan_onepass_body): each block reads every count before its chunk.
 constexpr uint32_t kOnePassPerThread = 16;
 
-// The density buffer of a persistent warp: what fits beside its staged chunk
-// in the room the pair lists take.
+// The density buffer of a persistent warp.  With its staged chunk it is the
+// largest member of the kernel's shared memory: 5,184 bytes per warp, the pair
+// lists take 3,072.
 constexpr uint32_t kDensCapPersist = 16;
 
 // One step's stages, from the hash (or, when the previous step hashed this
