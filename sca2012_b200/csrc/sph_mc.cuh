@@ -58,12 +58,11 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // kernel length when splat_with_kernel is set.
 //
 // One thread per two x-adjacent nodes (2m-1, 2m), or (QUAD) per 2 x 2 nodes,
-// (2m-1, 2m) in x and in y.  Nodes of one cell have one stencil: each of its
-// candidates is loaded once for all of them.  Each node still sums exactly its
-// own stencil's particles in its own walk order.  Nodes of more than one cell
-// are taken as x pairs, row after row (a node whose cell differs from its
-// partner's takes the candidates of the joint row range that fall in its own
-// range).
+// (2m-1, 2m) in x and in y, where all four lie in one cell.  Nodes of one cell
+// have one stencil: each of its candidates is loaded once for all of them.
+// Each node still sums exactly its own stencil's particles in its own walk
+// order (a node of a pair whose cell differs from its partner's takes the
+// candidates of the joint row range that fall in its own range).
 //
 // Bound by the candidates' loads (lanes of a warp read different cells, so a
 // 16-byte load is many L1 requests) and by issue: four nodes per load instead
@@ -72,15 +71,20 @@ inline int mc_alloc(McBuffers &mc, const sph_config &c, std::vector<void *> &all
 // us a step, built every tenth).
 constexpr uint32_t kSplatThreads = 128;
 
-// 2 x 2 nodes a thread where every group lies in one cell (an even number of
-// node spacings per cell in x and y; with 1, 3 or 5 the groups that straddle
-// cells run two rows in turn: 65 x 33 x 33 nodes 59 us with x pairs, 108 with
-// groups) and five blocks per SM are left (surface stage, x pairs / groups:
-// 2 spacings, 0.1M nodes 37 / 47 us, 0.3M 57 / 53, 0.8M 107 / 78; 4 spacings,
-// 0.3M 45 / 51, 0.8M 76 / 70, 6.4M 315 / 243).
+// 2 x 2 nodes a thread where every group lies in one cell and five blocks per
+// SM are left (surface stage, x pairs / groups: 2 spacings, 0.1M nodes 37 / 47
+// us, 0.3M 57 / 53, 0.8M 107 / 78; 4 spacings, 0.3M 45 / 51, 0.8M 76 / 70, 6.4M
+// 315 / 243).  With an even number s of node spacings per cell, cell q holds the
+// nodes q s + 1 .. q s + s, whole groups, and FP32 rounding moves none of them up
+// to 2^22 nodes an axis: the last one lies a part 1 / (nodes) of its value below
+// the next cell, and two roundings add less than a part 2^-23; the first one lies
+// (1 - q / ncell) / s above its cell's start, and rounding takes at most
+// (1 - q / ncell) ncell 2^-25 more than it would need to land on the start.  Such
+// an axis has an odd number of nodes, so no group is cut off.
 inline bool splat_quads(const uint32_t *ndens, const uint32_t *ncell, int num_sms)
 {
     return (ndens[0] - 1) % (2 * ncell[0]) == 0 && (ndens[1] - 1) % (2 * ncell[1]) == 0 &&
+           ndens[0] <= 1u << 22 && ndens[1] <= 1u << 22 &&
            (uint64_t)ndens[0] * ndens[1] * ndens[2] >= 4ull * 5 * kSplatThreads * num_sms;
 }
 
@@ -94,7 +98,7 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
                                                          const float4 *pos, float *dens)
 {
     dependent_entry();
-    const uint32_t R = c.ndens[0], Cn = c.ndens[1], L = c.ndens[2];
+    const uint32_t R = c.ndens[0], Cn = c.ndens[1];
     const uint32_t GX = R / 2 + 1, GY = QUAD ? Cn / 2 + 1 : Cn;
     const uint32_t G = splat_groups(c.ndens, QUAD);
     // per level: the squared splat radius and m * W's coefficient
@@ -106,28 +110,11 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
     for (uint32_t g = grid_stride_start(); g < G; g += grid_stride()) {
         const uint32_t gx = g % GX, gyz = g / GX, gy = gyz % GY, vz = gyz / GY;
         const uint32_t va = 2u * gx - 1u, vb = 2u * gx;   // va is not a node when gx = 0
-        const uint32_t ya = QUAD ? 2u * gy - 1u : gy, yb = 2u * gy;   // 2 gy - 1 is not a node when gy = 0
-        const bool has_b = vb < R, has_yb = QUAD && yb < Cn;
-        float *const row_a = dens + ((size_t)vz * Cn + ya) * R, *const row_b = dens + ((size_t)vz * Cn + yb) * R;
-        if (gx == 0 || gy == 0 || vz == 0) {
-            if (!QUAD || gy > 0) {
-                if (gx > 0) row_a[va] = 0.0f;
-                if (has_b) row_a[vb] = 0.0f;
-            }
-            if (has_yb) {   // row 0 is a face; above it only the nodes of a face
-                if (gx > 0) row_b[va] = 0.0f;
-                if (has_b) row_b[vb] = 0.0f;
-            }
-            continue;
-        }
         auto cell = [&](uint32_t v, int a) {
             return min((uint32_t)floorf(__fmul_rn(__fdiv_rn((float)v, (float)c.ndens[a]), (float)c.ncell[a])),
                        c.ncell[a] - 1);
         };
-        const uint32_t qax = cell(va, 0), qbx = has_b ? cell(vb, 0) : qax;
-        const uint32_t qya = cell(ya, 1), qyb = has_yb ? cell(yb, 1) : qya, qz = cell(vz, 2);
         const float xa = __fmul_rn((float)va, c.den_size), xb = __fmul_rn((float)vb, c.den_size);
-        const float nya = __fmul_rn((float)ya, c.den_size), nyb = __fmul_rn((float)yb, c.den_size);
         const float nz = __fmul_rn((float)vz, c.den_size);
         // acc += (m * W) * (rad^2 - r^2)^3 over r^2 < rad^2
         auto add = [&](float &acc, float nx, float ny, const float4 &pj, bool l1) {
@@ -137,60 +124,65 @@ __global__ void __launch_bounds__(kSplatThreads) k_splat(sph_config c, const uin
             const float x = __fsub_rn(rad2, r2);
             if (r2 < rad2) acc = __fmaf_rn(l1 ? cf0 : cf1, __fmul_rn(__fmul_rn(x, x), x), acc);
         };
-        if (QUAD && qbx == qax && qyb == qya) {   // one stencil for all four
-            const uint3 q = make_uint3(qax, qya, qz);
-            float aa = 0.0f, ba = 0.0f, ab = 0.0f, bb = 0.0f;
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy) {
-                    uint32_t b, e;
-                    if (!row_range<3>(c, off, q, dy, dz, b, e)) continue;
-                    for (uint32_t t = b; t < e; ++t) {
-                        const float4 pj = pos[t];
-                        const bool l1 = pj.w == 1.0f;
-                        add(aa, xa, nya, pj, l1);
-                        add(ba, xb, nya, pj, l1);
-                        add(ab, xa, nyb, pj, l1);
-                        add(bb, xb, nyb, pj, l1);
-                    }
-                }
-            row_a[va] = aa;
-            if (has_b) row_a[vb] = ba;
-            if (has_yb) {
-                row_b[va] = ab;
-                if (has_b) row_b[vb] = bb;
-            }
-            continue;
-        }
-        for (int yi = 0; yi < (has_yb ? 2 : 1); ++yi) {
-            const float ny = yi ? nyb : nya;
-            const uint3 qa = make_uint3(qax, yi ? qyb : qya, qz), qb = make_uint3(qbx, qa.y, qz);
-            float acc_a = 0.0f, acc_b = 0.0f;
-            for (int dz = -1; dz <= 1; ++dz)
-                for (int dy = -1; dy <= 1; ++dy) {
-                    uint32_t ba, ea;
-                    if (!row_range<3>(c, off, qa, dy, dz, ba, ea)) continue;
-                    if (qbx == qax) {   // one stencil for both
-                        for (uint32_t t = ba; t < ea; ++t) {
+        const uint32_t ya = QUAD ? 2u * gy - 1u : gy, yb = 2u * gy;   // 2 gy - 1 is not a node when gy = 0
+        float *const row_a = dens + ((size_t)vz * Cn + ya) * R;
+        if constexpr (QUAD) {
+            float *const row_b = dens + ((size_t)vz * Cn + yb) * R;
+            float aa = 0.0f, ba = 0.0f, ab = 0.0f, bb = 0.0f;   // 0 on the lower faces
+            if (gx > 0 && gy > 0 && vz > 0) {
+                const uint3 q = make_uint3(cell(va, 0), cell(ya, 1), cell(vz, 2));
+                const float nya = __fmul_rn((float)ya, c.den_size), nyb = __fmul_rn((float)yb, c.den_size);
+                for (int dz = -1; dz <= 1; ++dz)
+                    for (int dy = -1; dy <= 1; ++dy) {
+                        uint32_t b, e;
+                        if (!row_range<3>(c, off, q, dy, dz, b, e)) continue;
+                        for (uint32_t t = b; t < e; ++t) {
                             const float4 pj = pos[t];
                             const bool l1 = pj.w == 1.0f;
-                            add(acc_a, xa, ny, pj, l1);
-                            add(acc_b, xb, ny, pj, l1);
+                            add(aa, xa, nya, pj, l1);
+                            add(ba, xb, nya, pj, l1);
+                            add(ab, xa, nyb, pj, l1);
+                            add(bb, xb, nyb, pj, l1);
                         }
-                        continue;
                     }
-                    // node b's row range starts and ends later in slot order
-                    uint32_t bb, eb;
-                    row_range<3>(c, off, qb, dy, dz, bb, eb);
-                    for (uint32_t t = ba; t < eb; ++t) {
-                        const float4 pj = pos[t];
-                        const bool l1 = pj.w == 1.0f;
-                        if (t < ea) add(acc_a, xa, ny, pj, l1);
-                        if (t >= bb) add(acc_b, xb, ny, pj, l1);
+            }
+            if (gx > 0 && gy > 0) row_a[va] = aa;
+            if (gy > 0) row_a[vb] = ba;
+            if (gx > 0) row_b[va] = ab;
+            row_b[vb] = bb;
+        } else {
+            const bool has_b = vb < R;
+            float acc_a = 0.0f, acc_b = 0.0f;
+            if (gx > 0 && gy > 0 && vz > 0) {
+                const uint32_t qax = cell(va, 0), qbx = has_b ? cell(vb, 0) : qax;
+                const uint3 qa = make_uint3(qax, cell(gy, 1), cell(vz, 2)), qb = make_uint3(qbx, qa.y, qa.z);
+                const float ny = __fmul_rn((float)gy, c.den_size);
+                for (int dz = -1; dz <= 1; ++dz)
+                    for (int dy = -1; dy <= 1; ++dy) {
+                        uint32_t ba, ea;
+                        if (!row_range<3>(c, off, qa, dy, dz, ba, ea)) continue;
+                        if (qbx == qax) {   // one stencil for both
+                            for (uint32_t t = ba; t < ea; ++t) {
+                                const float4 pj = pos[t];
+                                const bool l1 = pj.w == 1.0f;
+                                add(acc_a, xa, ny, pj, l1);
+                                add(acc_b, xb, ny, pj, l1);
+                            }
+                            continue;
+                        }
+                        // node b's row range starts and ends later in slot order
+                        uint32_t bb, eb;
+                        row_range<3>(c, off, qb, dy, dz, bb, eb);
+                        for (uint32_t t = ba; t < eb; ++t) {
+                            const float4 pj = pos[t];
+                            const bool l1 = pj.w == 1.0f;
+                            if (t < ea) add(acc_a, xa, ny, pj, l1);
+                            if (t >= bb) add(acc_b, xb, ny, pj, l1);
+                        }
                     }
-                }
-            float *const row = yi ? row_b : row_a;
-            row[va] = acc_a;
-            if (has_b) row[vb] = acc_b;
+            }
+            if (gx > 0) row_a[va] = acc_a;
+            if (has_b) row_a[vb] = acc_b;
         }
     }
 }
