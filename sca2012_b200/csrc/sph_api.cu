@@ -196,10 +196,12 @@ bool scan_as_cluster(const sph_handle *h, uint32_t len) { return h->scan_cluster
 // that after one step: the rule goes by the count the host last knew, and the
 // bound only limits what a count grown unseen since then can cost.  Cluster
 // against full grid, split ranks with flags: 12.3 against 13.3 us at 262,144
-// particles, 18.4 / 15.4 at 589,824, 25.6 / 17.4 at 1,048,576, 71.7 / 33 at 4.2M;
-// a step without flags only checks their count, 6.1 / 9.2 at any size.  The line
-// lies where the one loses with flags what it gains without.
-constexpr uint32_t kClusterRankMax = 9u << 16, kClusterRankBound = 1u << 22;
+// particles, 18.4 / 15.4 at 589,824, 25.6 / 17.4 at 1.05M, 33.3 / 19.5 at 1.57M,
+// 41 / 21.5 at 2.1M, 71.7 / 33 at 4.2M; a step without flags only checks their
+// count, 6.1 / 9.2 at any size.  Of the scans of the 200-step four-way dam break
+// of 1.11M particles one in six has flags (one in twelve of the 500-step two-way
+// one): the line lies where that one loses what the other five gain.
+constexpr uint32_t kClusterRankMax = 3u << 19, kClusterRankBound = 1u << 22;
 
 bool ranks_as_cluster(const sph_handle *h)
 {

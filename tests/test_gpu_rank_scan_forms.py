@@ -11,7 +11,7 @@ from sca2012_b200 import scenes
 pytestmark = pytest.mark.gpu
 
 STATE = ("pos", "vel", "ev", "acc", "dens", "press", "energy", "surface", "level", "interior", "sibling")
-LIMIT = 9 << 16           # live count up to which the ranks are scanned by a cluster
+LIMIT = 3 << 19           # live count up to which the ranks are scanned by a cluster
 BOUND = 1 << 22           # and the largest bound at which they are
 CLUSTER, LAUNCHES = 2, 4  # launches of the split and the removal ranks of a step
 
@@ -43,7 +43,7 @@ def _plain_launches(cfg, st):
     return n + 1
 
 
-@pytest.mark.parametrize("counts,form", [((96, 96, 64), CLUSTER), ((96, 96, 65), LAUNCHES)])
+@pytest.mark.parametrize("counts,form", [((128, 128, 96), CLUSTER), ((128, 128, 97), LAUNCHES)])
 def test_form_follows_the_count(gpu, counts, form):
     """Counts on both sides of the limit, bounds (twice the count after a step) beyond it."""
     n = int(np.prod(counts))
