@@ -193,20 +193,17 @@ bool scan_as_cluster(const sph_handle *h, uint32_t len) { return h->scan_cluster
 
 // Whether the ranks of a step's flags are scanned by one cluster.  A scan reads
 // as many elements as particles live, while the host's bound may be four times
-// that after one step: the rule goes by the count the host last knew, and the
-// bound only limits what a count grown unseen since then can cost.  Cluster
+// that after one step, so the rule goes by the count the host last knew (one
+// grown unseen since then costs up to 2 % of a step, at any size).  Cluster
 // against full grid, split ranks with flags: 12.3 against 13.3 us at 262,144
 // particles, 18.4 / 15.4 at 589,824, 25.6 / 17.4 at 1.05M, 33.3 / 19.5 at 1.57M,
 // 41 / 21.5 at 2.1M, 71.7 / 33 at 4.2M; a step without flags only checks their
 // count, 6.1 / 9.2 at any size.  Of the scans of the 200-step four-way dam break
 // of 1.11M particles one in six has flags (one in twelve of the 500-step two-way
 // one): the line lies where that one loses what the other five gain.
-constexpr uint32_t kClusterRankMax = 3u << 19, kClusterRankBound = 1u << 22;
+constexpr uint32_t kClusterRankMax = 3u << 19;
 
-bool ranks_as_cluster(const sph_handle *h)
-{
-    return h->scan_cluster > 0 && std::min(h->n_ub, h->n_seen) <= kClusterRankMax && h->n_ub <= kClusterRankBound;
-}
+bool ranks_as_cluster(const sph_handle *h) { return h->scan_cluster > 0 && h->n_seen <= kClusterRankMax; }
 
 // Launch key of the step: every stage's grid and block size and the form of
 // its rank scans (a captured graph is valid while it is unchanged).

@@ -1,7 +1,7 @@
 """The two forms of the rank scans of a step (one cluster, or two launches over
-a full grid) are chosen by the live count the host last knew, with a limit on
-the host's bound: on launches and on replayed graphs, and with the bits of the
-persistent step, which has a scan of its own, in either form."""
+a full grid) are chosen by the live count the host last knew: by launches and by
+a handle that replays captured steps, with the bits of the persistent step,
+which has a scan of its own, in either form."""
 import numpy as np
 import pytest
 
@@ -12,7 +12,6 @@ pytestmark = pytest.mark.gpu
 
 STATE = ("pos", "vel", "ev", "acc", "dens", "press", "energy", "surface", "level", "interior", "sibling")
 LIMIT = 3 << 19           # live count up to which the ranks are scanned by a cluster
-BOUND = 1 << 22           # and the largest bound at which they are
 CLUSTER, LAUNCHES = 2, 4  # launches of the split and the removal ranks of a step
 
 
@@ -43,37 +42,39 @@ def _plain_launches(cfg, st):
     return n + 1
 
 
-@pytest.mark.parametrize("counts,form", [((128, 128, 96), CLUSTER), ((128, 128, 97), LAUNCHES)])
-def test_form_follows_the_count(gpu, counts, form):
-    """Counts on both sides of the limit, bounds (twice the count after a step) beyond it."""
-    n = int(np.prod(counts))
-    assert (n <= LIMIT) == (form == CLUSTER)
-    cfg, st = _setup(counts, 2 * n)
-    base = _plain_launches(cfg, st)
-    outs = []
-    for persistent in (False, True):
-        s = sph.Solver(cfg)
-        s.set_persistent(persistent)
-        s.set_state(st)
-        for k in range(4):
-            s.step(1)
-            if not persistent and k:   # the first step also hashes the new state
-                assert s.last_launch_count() == base + form
+@pytest.mark.parametrize("mode", ["launches", "graph"])
+def test_form_follows_the_count(gpu, mode):
+    """One handle stepped from counts on both sides of the limit (its bound is
+    beyond it after a step of either), and the persistent step beside it."""
+    cfg, big = _setup((128, 128, 97), 2 * 128 * 128 * 97)
+    n = 128 * 128 * 96
+    assert n == LIMIT
+    small = {k: v[:n] for k, v in big.items()}
+    base = _plain_launches(cfg, small)
+    s, p = sph.Solver(cfg), sph.Solver(cfg)
+    s.set_graph(mode == "graph")
+    p.set_persistent(True)
+    for st, form in ((big, LAUNCHES), (small, CLUSTER), (big, LAUNCHES)):
+        for h in (s, p):
+            h.set_state(st)
+            for k in range(3):
+                h.step(1)
+                if h is s and k:   # the first step also hashes the new state
+                    assert h.last_launch_count() == base + form
+            assert h.sync_status() == 0
         stats = s.last_step_stats()
-        assert s.sync_status() == 0
-        outs.append((stats, s.get_state()))
-        s.close()
-    (sa, xa), (sb, xb) = outs
-    assert sa == sb and sa["n_level2"] > 0
-    for f in STATE:
-        assert xa[f].tobytes() == xb[f].tobytes(), f
+        assert stats == p.last_step_stats() and stats["n_level2"] > 0
+        a, b = s.get_state(), p.get_state()
+        for f in STATE:
+            assert a[f].tobytes() == b[f].tobytes(), f
+    s.close()
+    p.close()
 
 
 @pytest.mark.parametrize("mode", ["launches", "graph"])
-def test_bound_limits_the_form(gpu, mode):
-    """A small count whose bound grows past its limit unseen: the scans move to
-    launches, in a captured step too, with the same bits."""
-    cfg, st = _setup((20, 20, 10), BOUND + 1000, ways=4)
+def test_form_keeps_to_the_count_as_the_bound_grows(gpu, mode):
+    """The bound of a small count grows past the limit unseen: still one cluster."""
+    cfg, st = _setup((20, 20, 10), 4 << 20, ways=4)
     base = _plain_launches(cfg, st)
     outs = []
     for m in (mode, "persistent"):
@@ -81,15 +82,12 @@ def test_bound_limits_the_form(gpu, mode):
         s.set_graph(m == "graph")
         s.set_persistent(m == "persistent")
         s.set_state(st)
-        bound = len(st["pos"])
         for k in range(8):
             s.step(1)
             if m != "persistent" and k:
-                assert s.last_launch_count() == base + (CLUSTER if bound <= BOUND else LAUNCHES), k
-            bound = min(4 * bound, cfg.max_particle)
-        stats = s.last_step_stats()
-        assert bound > BOUND and s.sync_status() == 0
-        outs.append((stats, s.get_state()))
+                assert s.last_launch_count() == base + CLUSTER, k
+        outs.append((s.last_step_stats(), s.get_state()))
+        assert s.sync_status() == 0
         s.close()
     (sa, xa), (sb, xb) = outs
     assert sa == sb and sa["n_end"] > len(st["pos"])
