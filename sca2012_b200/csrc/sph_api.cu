@@ -349,9 +349,9 @@ void scan_u32(sph_handle *h, uint32_t *in, uint32_t *out, uint32_t len, uint32_t
                                                       clear ? 1 : 0});
         return;
     }
-    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, nullptr, len, h->scan_blocks);
-    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, nullptr, len, h->scan_blocks, grand,
-                                                                        total_at_len, nullptr);
+    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, len, h->scan_blocks);
+    scan_phase23<uint32_t><<<kScanBlocks, kScanThreads, 0, h->stream>>>(in, out, len, h->scan_blocks, grand,
+                                                                        total_at_len);
     h->last_launches += 2;
     if (clear) cudaMemsetAsync(in, 0, sizeof(uint32_t) * len, h->stream);
 }

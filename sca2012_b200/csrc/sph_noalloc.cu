@@ -181,7 +181,7 @@ extern "C" int sph_sort_cells_noalloc(const sph_config *cfg, uint32_t n, const f
     cudaMemsetAsync(count, 0, sizeof(uint32_t) * (nc + 1), s);   // counts start at zero every call
     if (cfg->dim == 3) na_hash<3><<<G, kThreads, 0, s>>>(*cfg, n, pos_dev, key, slot, count);
     else na_hash<2><<<G, kThreads, 0, s>>>(*cfg, n, pos_dev, key, slot, count);
-    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, s>>>(count, nullptr, nc, blocks);
+    scan_phase1<uint32_t><<<kScanBlocks, kScanThreads, 0, s>>>(count, nc, blocks);
     scan_phase2<uint32_t><<<1, kScanBlocks, 0, s>>>(blocks, grand);
     scan_phase3<uint32_t><<<kScanBlocks, kScanThreads, 0, s>>>(count, off, nullptr, nc, blocks, grand, 1, nullptr);
     na_scatter<<<G, kThreads, 0, s>>>(n, key, slot, off, tmp);

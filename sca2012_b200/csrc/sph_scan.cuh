@@ -90,10 +90,10 @@ __device__ __forceinline__ void scan_phase1_body(const T *in, uint32_t len, T *b
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kScanThreads) scan_phase1(const T *__restrict__ in, const uint32_t *len_ptr,
-                                                           uint32_t len_const, T *__restrict__ block_tot)
+__global__ void __launch_bounds__(kScanThreads) scan_phase1(const T *__restrict__ in, uint32_t len,
+                                                           T *__restrict__ block_tot)
 {
-    scan_phase1_body<T>(in, len_ptr ? *len_ptr : len_const, block_tot);
+    scan_phase1_body<T>(in, len, block_tot);
 }
 
 // Exclusive scan of nb block totals by one block of any size (each thread
@@ -241,11 +241,10 @@ __device__ __forceinline__ void scan_onepass_body(const T *in, T *out, uint32_t 
 // Phases 2 and 3 as one launch (after scan_phase1 over the same grid).
 template <typename T>
 __global__ void __launch_bounds__(kScanThreads) scan_phase23(const T *__restrict__ in, T *__restrict__ out,
-                                                            const uint32_t *len_ptr, uint32_t len_const,
-                                                            const T *__restrict__ block_tot, T *grand,
-                                                            int out_total_at_len, uint32_t *list)
+                                                            uint32_t len, const T *__restrict__ block_tot,
+                                                            T *grand, int out_total_at_len)
 {
-    scan_phase23_body<T>(in, out, len_ptr ? *len_ptr : len_const, block_tot, grand, out_total_at_len, list);
+    scan_phase23_body<T>(in, out, len, block_tot, grand, out_total_at_len, nullptr);
 }
 
 // ------------------------------------------------------------ one-launch scan
